@@ -473,6 +473,10 @@ int hrn_set_mesh(hrn_ctx *c, int32_t nj, int32_t nel, int32_t neq, const double 
         if (mtel[e] != 1 && mtel[e] != 2) return set_error(c, HRN_EARG, "MTEL must be 1 (RD) or 2 (PML)");
     cudaSetDevice(c->device);
     c->have_elem = false;
+    c->have_line = false;
+    c->line_epoch = 0;
+    if (is_line_variant(c->lanes_f)) c->lanes_f = 0;   // the new mesh may not suit the line operator: tune again
+    if (is_line_variant(c->lanes_a)) c->lanes_a = 0;
     c->op_from_mesh = false;
     c->nj = nj;
     c->nel = nel;
@@ -745,7 +749,8 @@ int hrn_get_state(hrn_ctx *c, int32_t step, int32_t shot, double *x1, double *x2
     for (int k = 0; k < 3; ++k) {
         if (!out[k]) continue;
         for (int i = 0; i < c->neq; ++i) {
-            const size_t at = size_t(k) * vn + size_t(i) * S + size_t(shot);
+            const size_t row = is_line_variant(c->fwd_variant) ? size_t(c->line_row[i]) : size_t(i);
+            const size_t at = size_t(k) * vn + row * S + size_t(shot);
             out[k][i] = c->precision == HRN_FP64 ? reinterpret_cast<const double *>(h.data())[at]
                                                  : double(reinterpret_cast<const float *>(h.data())[at]);
         }
@@ -854,12 +859,12 @@ int hrn_set_variant(hrn_ctx *c, int32_t forward, int32_t adjoint)
     ++c->epoch;
     auto ok = [](int v) {
         return v == 0 || v == 40 || v == 80 || v == 160 || v == 41 || v == 81 || v == 161 || v == 42 || v == 43 || v == 82 ||
-               v == 83 || hrn::is_gt_variant(v) || (v >= 90 && v <= 95) || (v >= 100 && v <= 105);
+               v == 83 || hrn::is_gt_variant(v) || (v >= 90 && v <= 98) || (v >= 100 && v <= 105);
     };
     if (!ok(forward) || !ok(adjoint))
         return set_error(c, HRN_EARG, "variant must be 0 (tune), lanes*10 + mat + tiled (lanes 4/8/16, mat 0/1, tiled 0/2/4; "
                                       "tiled only with lanes 4/8) or 90-95 / 100-105 (matrix-free with materialized / rebuilt stage inputs: "
-                                      "slots even, atomics odd; 1, 2, 4 shots per thread)");
+                                      "slots even, atomics odd; 1, 2, 4 shots per thread) or 96-98 (line operator)");
     c->lanes_f = forward;
     c->lanes_a = adjoint;
     return HRN_OK;

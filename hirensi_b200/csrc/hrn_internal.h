@@ -183,6 +183,23 @@ struct hrn_ctx {
     hrn::DevBuf d_eslots;         // [P * 27][9][S] element contributions (T)
     hrn::DevBuf d_eacc;           // [neq][S] row accumulator of the atomic variant (T), kept zero between stages
 
+    // line-operator stage (variants 96-98): tables of the mesh, see hrn_line.cuh
+    bool have_line = false;
+    int line_ok = 0;              // 1: the mesh suits it, -1: it does not
+    int line_box = 0;             // every regular-domain element is an axis-aligned box
+    int line_npn = 0, line_nup = 0, line_nun = 0;   // PML nodes; displacement nodes in the PML, all
+    int line_wd = 0, line_wt = 0;
+    int line_stress_src = 0, line_stress_hist = 0;
+    uint64_t line_epoch = 0;      // settings epoch of the two flags and of the row lists below
+    std::vector<int32_t> line_row;               // [neq] state row of an equation
+    hrn::DevBuf d_line_row, d_line_store_row, d_line_rec_row;
+    hrn::DevBuf d_line_pnode, d_line_didx, d_line_dcf, d_line_pcoef;
+    hrn::DevBuf d_line_unode, d_line_ucoef, d_line_uim, d_line_tidx, d_line_tcf, d_line_ridx;
+    hrn::DevBuf d_line_rpt, d_line_rgeo;
+    hrn::DevBuf d_line_rslot;     // [27][3][nel_rd][S] regular-domain element contributions (T)
+    hrn::DevBuf d_line_P;         // [1 or 2 sets][3][9][npn][S] P of this and the next stage, Z (T)
+    int fwd_variant = 0;          // variant of the forward whose states the checkpoints hold
+
     // ---- history
     int nstore = 0;
     std::vector<int32_t> h_store_eq;
@@ -312,6 +329,13 @@ int elem_prepare(hrn_ctx *c);
 int elem_ready(hrn_ctx *c);
 int elem_stage(hrn_ctx *c, const void *stage_args, int stage, int adj, int acc, int shots_per_thread, int mat);
 bool elem_variant_valid(const hrn_ctx *c, int variant);
+// line-operator stage: 96, 97, 98 = up to 1, 2, 4 shots per thread (the most that divides
+// the shot count; 4 in FP32 only), so each serves any shot count
+inline bool is_line_variant(int v) { return v >= 96 && v <= 98; }
+int line_ready(hrn_ctx *c, int *ok);
+int line_stage(hrn_ctx *c, const void *stage_args, int stage, int adj, int variant, int first, bool pdl);
+int line_stage_f64(hrn_ctx *c, const void *stage_args, int stage, int adj, int sv, int first, bool pdl);
+int line_stage_f32(hrn_ctx *c, const void *stage_args, int stage, int adj, int sv, int first, bool pdl);
 int vec_axpby(hrn_ctx *c, int n, double a, const double *x, double b, const double *y, double *z);
 int set_error(hrn_ctx *c, int code, const std::string &msg);
 int cuda_error(hrn_ctx *c, cudaError_t e, const char *what);

@@ -1,0 +1,446 @@
+// hrn_line.cu -- tables of the line-operator stage (hrn_line.cuh): the nodal
+// derivative operators D_x, D_y, D_z of the PML and their transposes, the PML
+// coefficients of every node, and the regular-domain element tables.  All of
+// them depend on the mesh alone, so they are built once per mesh.
+#include <cuda_runtime.h>
+#include <stdint.h>
+#include <thrust/execution_policy.h>
+#include <thrust/device_ptr.h>
+#include <thrust/functional.h>
+#include <thrust/reduce.h>
+
+#include <algorithm>
+#include <cmath>
+#include <vector>
+
+#include "hrn_internal.h"
+
+namespace hrn {
+
+constexpr int kLineNb = 32;        // most nodes that share a grid line through one node (13 on structured meshes)
+constexpr int kLineBuildThreads = 32;
+constexpr int kLineCoefPlanes = 15;
+// Entries below this share of their node's largest one are rounding residue of opposite
+// contributions (the one-sided derivatives at a node between two equal elements).
+constexpr double kLineDrop = 16 * 2.2204460492503131e-16;
+// PML weights that differ by less along a line are the same value with rounding.
+constexpr double kWeightTol = 1e-13;
+// An element counts as an axis-aligned box when its DJI and detJ vary by less than this.
+constexpr double kBoxTol = 1e-13;
+
+__device__ __forceinline__ double gll_d(int a, int b)   // l_b'(xi_a)
+{
+    return a == 0 ? (b == 0 ? -1.5 : (b == 1 ? 2.0 : -0.5))
+                  : (a == 1 ? (b == 0 ? -0.5 : (b == 1 ? 0.0 : 0.5)) : (b == 0 ? 0.5 : (b == 1 ? -2.0 : 1.5)));
+}
+
+// Entries of row r of D_k (TR = 0: PML node J, columns the nodes on its lines) or of
+// D_k^T (TR = 1: displacement node I, columns the PML nodes J whose lines pass it), at
+// most w a direction (TR = 0) or a row (TR = 1).  idx == null: count them, per direction
+// into cnt[3 r + k] or per row into cnt[r]; else write them, entry u of a direction at
+// idx[(k w + u) nrow + r], of a row at idx[u nrow + r], divided by fj = F j0 of node J.
+template <typename T, int TR>
+__global__ void __launch_bounds__(kLineBuildThreads)
+k_line_entries(int nrow, const int32_t *__restrict__ nodes, const int32_t *__restrict__ nptr, const uint32_t *__restrict__ nslot,
+               int nel_pml, const int32_t *__restrict__ el_node, const double *__restrict__ geom,
+               const int32_t *__restrict__ target, int ntarget, const double *__restrict__ pmlw, const double *__restrict__ fj, int w,
+               int32_t *__restrict__ cnt, int32_t *__restrict__ idx, T *__restrict__ cf, int *__restrict__ bad)
+{
+    __shared__ int32_t s_nb[kLineNb][kLineBuildThreads];
+    __shared__ double s_cf[3][kLineNb][kLineBuildThreads];
+    const int r = blockIdx.x * kLineBuildThreads + threadIdx.x, th = threadIdx.x;
+    if (r >= nrow) return;
+    const int node = nodes[r];
+    int n = 0;
+    for (int s = nptr[node]; s < nptr[node + 1]; ++s) {
+        const uint32_t sl = nslot[s] & 0x7fffffffu;
+        const int p = int(sl / 27), q = int(sl % 27);
+        if (p >= nel_pml) continue;   // regular-domain elements follow the PML's
+        const int qm[3] = {q % 3, (q / 3) % 3, q / 9};
+        const int str[3] = {1, 3, 9};
+        for (int m = 0; m < 3; ++m)
+            for (int t = 0; t < 3; ++t) {
+                const int o = q + (t - qm[m]) * str[m];
+                const int nb = el_node[size_t(p) * 27 + o];
+                // the derivative at point J = q (TR 0) or J = o (TR 1) of the node at the other
+                const double *g = geom + (size_t(p) * 27 + (TR ? o : q)) * 10;
+                const double d = g[9] * (TR ? gll_d(t, qm[m]) : gll_d(qm[m], t));
+                int k = 0;
+                while (k < n && s_nb[k][th] != nb) ++k;
+                if (k == n) {
+                    if (n == kLineNb) { atomicExch(bad, 1); return; }
+                    s_nb[n][th] = nb;
+                    for (int x = 0; x < 3; ++x) s_cf[x][n][th] = 0.0;
+                    ++n;
+                }
+                for (int x = 0; x < 3; ++x) s_cf[x][k][th] += d * g[3 * m + x];
+            }
+    }
+    double top = 0.0;
+    for (int k = 0; k < n; ++k)
+        for (int x = 0; x < 3; ++x) top = fmax(top, fabs(s_cf[x][k][th]));
+    int at = 0;
+    for (int x = 0; x < 3; ++x) {
+        if (!TR) at = 0;
+        for (int k = 0; k < n; ++k) {
+            const int nb = s_nb[k][th], to = target[nb];
+            if (to < 0 || !(fabs(s_cf[x][k][th]) > kLineDrop * top)) continue;
+            if (idx) {
+                const size_t o = (size_t(TR ? 0 : x) * w + at) * nrow + r;
+                idx[o] = TR ? 3 * ntarget * x + to : to;
+                cf[o] = T(s_cf[x][k][th] / fj[TR ? to : r]);
+                // the weights of direction x have to be the same at both ends of the entry
+                for (int t = 0; t < 3; ++t) {
+                    const double wn = pmlw[size_t(node) * 12 + 3 * t + x], wb = pmlw[size_t(nb) * 12 + 3 * t + x];
+                    if (!(fabs(wn - wb) <= kWeightTol * fabs(wn))) atomicExch(bad, 2);
+                }
+            }
+            ++at;
+        }
+        if (!idx && !TR) cnt[3 * r + x] = at;
+    }
+    if (!idx && TR) cnt[r] = at;
+}
+
+// Coefficient planes of the PML nodes' stress rows (disp = 0) or of the displacement
+// nodes (disp = 1), summed over a node's PML elements; eq: first equation of its rows.
+template <typename T>
+__global__ void k_line_coef(int n, int disp, const int32_t *__restrict__ ids, const int32_t *__restrict__ eqs,
+                            const int32_t *__restrict__ nptr, const uint32_t *__restrict__ nslot, int nel_pml,
+                            const double *__restrict__ geom, const double *__restrict__ rho, const double *__restrict__ pmlw,
+                            const double *__restrict__ im, double j0, T *__restrict__ out)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    const int node = ids[r];
+    double F = 0.0;
+    for (int s = nptr[node]; s < nptr[node + 1]; ++s) {
+        const uint32_t sl = nslot[s] & 0x7fffffffu;
+        const int p = int(sl / 27);
+        if (p >= nel_pml) continue;
+        const double f0 = geom[size_t(sl) * 10 + 9];
+        F += disp ? rho[p] * f0 : f0;
+    }
+    const double *w = pmlw + size_t(node) * 12;
+    auto put = [&](int i, double v) { out[size_t(i) * n + r] = T(v); };
+    const int eq = eqs[r];
+    const double fj = disp ? 1.0 : F * j0;
+    for (int k = 0; k < 9; ++k) put(k, fj * w[k]);
+    for (int t = 0; t < 3; ++t) put(9 + t, -im[eq] * F * w[9 + t]);
+    put(12, disp ? 0.0 : -im[eq] * fj);
+    put(13, disp ? 0.0 : -im[eq + 3] * fj);
+    put(14, (w[6] != 0.0 || w[7] != 0.0 || w[8] != 0.0 || F * w[11] != 0.0) ? 1.0 : 0.0);
+}
+
+__global__ void k_line_uim(int n, const int4 *__restrict__ unode, const double *__restrict__ im, double *__restrict__ out)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < n) out[r] = -im[unode[r].x];
+}
+
+// F j0 of the PML nodes: the sum of w detJ over a node's PML elements times j0.
+__global__ void k_line_fj(int n, const int32_t *__restrict__ ids, const int32_t *__restrict__ nptr, const uint32_t *__restrict__ nslot,
+                          int nel_pml, const double *__restrict__ geom, double j0, double *__restrict__ out)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    double F = 0.0;
+    for (int s = nptr[ids[r]]; s < nptr[ids[r] + 1]; ++s) {
+        const uint32_t sl = nslot[s] & 0x7fffffffu;
+        if (int(sl / 27) < nel_pml) F += geom[size_t(sl) * 10 + 9];
+    }
+    out[r] = F * j0;
+}
+
+// State rows of a list of equations.
+__global__ void k_line_rows(int n, const int32_t *__restrict__ row, const int32_t *__restrict__ eq, int32_t *__restrict__ out)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) out[i] = row[eq[i]];
+}
+
+// Axis-aligned boxes: DJI diagonal and the same, like detJ, at all 27 points.
+__global__ void k_line_box(int nrd, const double *__restrict__ geom, int *__restrict__ bad)
+{
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= nrd * 27) return;
+    const double *g = geom + size_t(t) * 10, *c = geom + (size_t(t / 27) * 27 + 13) * 10;
+    const int q = t % 27;
+    auto w = [](int a) { return a == 1 ? 4.0 / 3.0 : 1.0 / 3.0; };
+    const double wq = w(q % 3) * w((q / 3) % 3) * w(q / 9), wc = 64.0 / 27.0;
+    bool ok = fabs(g[9] * wc - c[9] * wq) <= kBoxTol * c[9] * wq;
+    double dmin = fmin(fabs(c[0]), fmin(fabs(c[4]), fabs(c[8])));
+    for (int m = 0; m < 3; ++m)
+        for (int k = 0; k < 3; ++k) {
+            const double v = g[3 * m + k];
+            ok = ok && (m == k ? fabs(v - c[4 * m]) <= kBoxTol * fabs(c[4 * m]) : fabs(v) <= kBoxTol * dmin);
+        }
+    if (!ok) atomicExch(bad, 1);
+}
+
+__global__ void k_line_rgeo(int64_t n, int box, const double *__restrict__ geom, double *__restrict__ out)
+{
+    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (t >= n) return;
+    if (box) {
+        const double *c = geom + (size_t(t / 4) * 27 + 13) * 10;   // the centre point, weight 64/27
+        const int k = int(t % 4);
+        out[t] = k == 0 ? c[4] / c[0] : (k == 1 ? c[8] / c[0] : (k == 2 ? c[9] / (64.0 / 27.0) * c[0] * c[0] : 0.0));
+    } else {
+        out[t] = geom[t];
+    }
+}
+
+// Entry planes of D (TR = 0) or D^T (TR = 1): *w entries a direction or a row.
+template <typename T, int TR>
+static int build_entries(hrn_ctx *c, int nrow, const DevBuf &nodes, const DevBuf &target, const DevBuf &fj, int *w, DevBuf &idx, DevBuf &cf, DevBuf &bad)
+{
+    *w = 0;
+    if (nrow == 0) return 0;
+    DevBuf cnt;
+    const size_t nc = size_t(nrow) * (TR ? 1 : 3);
+    HRN_CUDA(c, cnt.alloc(nc * 4));
+    HRN_CUDA(c, cudaMemsetAsync(cnt.p, 0, cnt.bytes, c->stream));
+    const int nb = (nrow + kLineBuildThreads - 1) / kLineBuildThreads;
+    auto launch = [&](int32_t *out) {
+        k_line_entries<T, TR><<<nb, kLineBuildThreads, 0, c->stream>>>(
+            nrow, nodes.as<int32_t>(), c->d_nslot_ptr.as<int32_t>(), c->d_nslot.as<uint32_t>(), c->nel_pml_e,
+            c->d_el_node.as<int32_t>(), c->d_el_geom.as<double>(), target.as<int32_t>(), c->line_npn, c->d_pmlw.as<double>(), fj.as<double>(), *w,
+            cnt.as<int32_t>(), out, cf.as<T>(), bad.as<int>());
+        ++c->launches;
+        return cudaGetLastError();
+    };
+    HRN_CUDA(c, launch(nullptr));
+    thrust::device_ptr<int32_t> p(cnt.as<int32_t>());
+    *w = std::max(1, thrust::reduce(thrust::cuda::par.on(c->stream), p, p + nc, 0, thrust::maximum<int32_t>()));
+    const size_t n = nc * size_t(*w);
+    HRN_CUDA(c, idx.alloc(n * 4));
+    HRN_CUDA(c, cf.alloc(n * sizeof(T)));
+    HRN_CUDA(c, cudaMemsetAsync(idx.p, 0xff, n * 4, c->stream));   // -1: no entry
+    HRN_CUDA(c, cudaMemsetAsync(cf.p, 0, n * sizeof(T), c->stream));
+    HRN_CUDA(c, launch(idx.as<int32_t>()));
+    HRN_CUDA(c, cudaStreamSynchronize(c->stream));   // cnt is released here
+    return 0;
+}
+
+template <typename T>
+static int line_tables(hrn_ctx *c)
+{
+    const int nj = c->nj;
+    // equations of a node: three displacements in a row or none, six stresses in a row or none
+    std::vector<int32_t> ubase(nj), sbase(nj), pidx(nj, -1);
+    c->line_ok = -1;
+    if (c->neq >= (1 << 29)) return 0;   // 32-bit offsets into [neq][8 shots]
+    for (int j = 0; j < nj; ++j) {
+        const int32_t *id = c->h_id.data() + size_t(j) * 9;
+        ubase[j] = id[0];
+        sbase[j] = id[3];
+        for (int d = 1; d < 3; ++d)
+            if (id[d] != (id[0] < 0 ? -1 : id[0] + d)) return 0;
+        for (int d = 1; d < 6; ++d)
+            if (id[3 + d] != (id[3] < 0 ? -1 : id[3] + d)) return 0;
+    }
+    static const unsigned char ijk[27][3] = {{2, 0, 0}, {2, 2, 0}, {0, 2, 0}, {0, 0, 0}, {2, 0, 2}, {2, 2, 2}, {0, 2, 2},
+                                             {0, 0, 2}, {2, 1, 0}, {1, 2, 0}, {0, 1, 0}, {1, 0, 0}, {2, 0, 1}, {2, 2, 1},
+                                             {0, 2, 1}, {0, 0, 1}, {2, 1, 2}, {1, 2, 2}, {0, 1, 2}, {1, 0, 2}, {1, 1, 0},
+                                             {2, 1, 1}, {1, 2, 1}, {0, 1, 1}, {1, 0, 1}, {1, 1, 2}, {1, 1, 1}};
+    unsigned char node_at[27];
+    for (int i = 0; i < 27; ++i) node_at[9 * ijk[i][2] + 3 * ijk[i][1] + ijk[i][0]] = (unsigned char)i;
+    std::vector<unsigned char> kind(nj, 0);   // 1: in the PML, 2: in the regular domain
+    std::vector<int32_t> rptr(size_t(nj) + 1, 0);
+    for (int e = 0; e < c->nel; ++e)
+        for (int i = 0; i < 27; ++i) {
+            const int j = c->h_inod[size_t(e) * 27 + i];
+            kind[j] |= (unsigned char)c->h_mtel[e] == 2 ? 1 : 2;
+            if (c->h_mtel[e] == 1) rptr[j + 1]++;
+        }
+    for (int j = 0; j < nj; ++j) rptr[j + 1] += rptr[j];
+    std::vector<int32_t> rlist(std::max<size_t>(size_t(rptr[nj]), 1), 0), pos(rptr.begin(), rptr.end() - 1);
+    std::vector<int2> rpt(std::max<size_t>(size_t(c->nel_rd_e) * 27, 1));
+    int k = 0;
+    for (int e = 0; e < c->nel; ++e) {
+        if (c->h_mtel[e] != 1) continue;
+        for (int q = 0; q < 27; ++q) {
+            const int j = c->h_inod[size_t(e) * 27 + node_at[q]];
+            rpt[size_t(k) * 27 + q] = make_int2(j, -1);
+            rlist[pos[j]++] = k * 27 + q;
+        }
+        ++k;
+    }
+    // rows of the state: displacements [3][nun], then stresses [6][npn]
+    std::vector<int2> pnode;
+    std::vector<int32_t> pn_id, pn_eq, un_id, un_eq, unidx(nj, -1);
+    std::vector<int4> unode;
+    for (int j = 0; j < nj; ++j) {
+        if (!(kind[j] & 1)) {
+            if (sbase[j] >= 0) return 0;   // a stress unknown outside the PML
+            continue;
+        }
+        if (sbase[j] < 0) return 0;        // constrained stresses
+        pidx[j] = int32_t(pnode.size());
+        pnode.push_back(make_int2(j, sbase[j]));
+        pn_id.push_back(j);
+        pn_eq.push_back(sbase[j]);
+    }
+    int most = 0;
+    for (int pass = 0; pass < 2; ++pass) {
+        for (int j = 0; j < nj; ++j) {
+            if (ubase[j] < 0 || ((kind[j] & 1) != 0) != (pass == 0)) continue;
+            unidx[j] = int32_t(unode.size());
+            unode.push_back(make_int4(ubase[j], pidx[j], rptr[j + 1] - rptr[j], 0));
+            un_id.push_back(j);
+            un_eq.push_back(ubase[j]);
+            most = std::max(most, rptr[j + 1] - rptr[j]);
+        }
+        if (pass == 0) c->line_nup = int(unode.size());
+    }
+    const int nun = int(unode.size()), npn = int(pnode.size());
+    if (int64_t(3) * nun + int64_t(6) * npn != c->neq) return 0;   // every equation belongs to one node
+    if (most > kLineNb || nun == 0) return 0;
+    c->line_nun = nun;
+    c->line_npn = npn;
+    std::vector<int32_t> &row = c->line_row;
+    row.assign(size_t(c->neq), 0);
+    for (int u = 0; u < nun; ++u)
+        for (int d = 0; d < 3; ++d) row[size_t(un_eq[u]) + d] = d * nun + u;
+    for (int p = 0; p < npn; ++p)
+        for (int d = 0; d < 6; ++d) row[size_t(pn_eq[p]) + d] = 3 * nun + d * npn + p;
+    std::vector<int32_t> ridx(std::max<size_t>(size_t(most) * nun, 1), -1);
+    for (int u = 0; u < nun; ++u)
+        for (int k = rptr[un_id[u]]; k < rptr[un_id[u] + 1]; ++k) {
+            const int e = rlist[k] / 27, q = rlist[k] % 27;
+            ridx[size_t(k - rptr[un_id[u]]) * nun + u] = 3 * c->nel_rd_e * q + e;
+        }
+    for (auto &p : rpt) p.y = unidx[p.x];
+    std::vector<int32_t> zidx(pidx);   // records of Z: PML nodes whose displacements are free
+    for (int j = 0; j < nj; ++j)
+        if (ubase[j] < 0) zidx[j] = -1;
+    DevBuf d_pn, d_pe, d_un, d_ue, d_zi, d_pi, d_fj, bad;
+    auto put = [&](DevBuf &b, const void *src, size_t bytes) -> int {
+        HRN_CUDA(c, b.alloc(std::max<size_t>(bytes, 16)));
+        if (bytes) HRN_CUDA(c, cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, c->stream));
+        return 0;
+    };
+    if (int rc = put(c->d_line_pnode, pnode.data(), pnode.size() * 8)) return rc;
+    if (int rc = put(c->d_line_unode, unode.data(), unode.size() * 16)) return rc;
+    if (int rc = put(c->d_line_ridx, ridx.data(), ridx.size() * 4)) return rc;
+    if (int rc = put(c->d_line_rpt, rpt.data(), rpt.size() * 8)) return rc;
+    if (int rc = put(c->d_line_row, row.data(), row.size() * 4)) return rc;
+    if (int rc = put(d_pn, pn_id.data(), pn_id.size() * 4)) return rc;
+    if (int rc = put(d_pe, pn_eq.data(), pn_eq.size() * 4)) return rc;
+    if (int rc = put(d_un, un_id.data(), un_id.size() * 4)) return rc;
+    if (int rc = put(d_ue, un_eq.data(), un_eq.size() * 4)) return rc;
+    if (int rc = put(d_zi, zidx.data(), zidx.size() * 4)) return rc;
+    if (int rc = put(d_pi, pidx.data(), pidx.size() * 4)) return rc;
+    HRN_CUDA(c, bad.alloc(8));
+    HRN_CUDA(c, cudaMemsetAsync(bad.p, 0, 8, c->stream));
+    double j0 = 1.0;   // an inverse length of the PML's elements
+    if (npn > 0) {
+        double g[9];
+        HRN_CUDA(c, cudaMemcpyAsync(g, c->d_el_geom.p, sizeof(g), cudaMemcpyDeviceToHost, c->stream));
+        HRN_CUDA(c, cudaStreamSynchronize(c->stream));
+        for (double v : g)
+            if (v != 0.0) { j0 = std::fabs(v); break; }
+        HRN_CUDA(c, d_fj.alloc(size_t(npn) * 8));
+        k_line_fj<<<(npn + 127) / 128, 128, 0, c->stream>>>(npn, d_pn.as<int32_t>(), c->d_nslot_ptr.as<int32_t>(), c->d_nslot.as<uint32_t>(),
+                                                            c->nel_pml_e, c->d_el_geom.as<double>(), j0, d_fj.as<double>());
+        ++c->launches;
+        HRN_CUDA(c, cudaGetLastError());
+    }
+    if (int rc = build_entries<T, 0>(c, npn, d_pn, d_zi, d_fj, &c->line_wd, c->d_line_didx, c->d_line_dcf, bad)) return rc;
+    if (int rc = build_entries<T, 1>(c, c->line_nup, d_un, d_pi, d_fj, &c->line_wt, c->d_line_tidx, c->d_line_tcf, bad)) return rc;
+    auto coef = [&](int n, int disp, const DevBuf &ids, const DevBuf &eqs, DevBuf &out) -> int {
+        HRN_CUDA(c, out.alloc(size_t(std::max(n, 1)) * kLineCoefPlanes * sizeof(T)));
+        if (n == 0) return 0;
+        k_line_coef<T><<<(n + 127) / 128, 128, 0, c->stream>>>(
+            n, disp, ids.as<int32_t>(), eqs.as<int32_t>(), c->d_nslot_ptr.as<int32_t>(), c->d_nslot.as<uint32_t>(), c->nel_pml_e,
+            c->d_el_geom.as<double>(), c->d_el_rho.as<double>(), c->d_pmlw.as<double>(), c->d_im.as<double>(), j0, out.as<T>());
+        ++c->launches;
+        HRN_CUDA(c, cudaGetLastError());
+        return 0;
+    };
+    if (int rc = coef(npn, 0, d_pn, d_pe, c->d_line_pcoef)) return rc;
+    if (int rc = coef(c->line_nup, 1, d_un, d_ue, c->d_line_ucoef)) return rc;
+    HRN_CUDA(c, c->d_line_uim.alloc(size_t(nun) * 8));
+    k_line_uim<<<(nun + 255) / 256, 256, 0, c->stream>>>(nun, c->d_line_unode.as<int4>(), c->d_im.as<double>(), c->d_line_uim.as<double>());
+    ++c->launches;
+    HRN_CUDA(c, cudaGetLastError());
+    const double *rg = c->d_el_geom.as<double>() + size_t(c->nel_pml_e) * 270;
+    if (c->nel_rd_e > 0) {
+        k_line_box<<<(c->nel_rd_e * 27 + 255) / 256, 256, 0, c->stream>>>(c->nel_rd_e, rg, bad.as<int>() + 1);
+        ++c->launches;
+        HRN_CUDA(c, cudaGetLastError());
+    }
+    int flags[2];
+    HRN_CUDA(c, cudaMemcpyAsync(flags, bad.p, 8, cudaMemcpyDeviceToHost, c->stream));
+    HRN_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (flags[0]) return 0;   // too many nodes on the lines of one, or weights that vary along a line
+    c->line_box = flags[1] ? 0 : 1;
+    const int64_t ng = int64_t(c->nel_rd_e) * (c->line_box ? 4 : 270);
+    HRN_CUDA(c, c->d_line_rgeo.alloc(std::max<size_t>(size_t(ng), 1) * 8));
+    if (ng > 0) {
+        k_line_rgeo<<<unsigned((ng + 255) / 256), 256, 0, c->stream>>>(ng, c->line_box, rg, c->d_line_rgeo.as<double>());
+        ++c->launches;
+        HRN_CUDA(c, cudaGetLastError());
+    }
+    HRN_CUDA(c, cudaStreamSynchronize(c->stream));
+    c->line_ok = 1;
+    return 0;
+}
+
+// Tables of the current mesh; c->line_ok says whether the mesh suits the line operator.
+static int line_prepare(hrn_ctx *c)
+{
+    if (int rc = elem_prepare(c)) return rc;
+    if (c->have_line) return 0;
+    const int rc = c->precision == HRN_FP64 ? line_tables<double>(c) : line_tables<float>(c);
+    if (rc) return rc;
+    c->have_line = true;
+    return 0;
+}
+
+// Tables and buffers for the current shots; *ok = 0 when the mesh needs another variant.
+int line_ready(hrn_ctx *c, int *ok)
+{
+    *ok = 0;
+    if (!c->op_from_mesh) return 0;
+    if (int rc = line_prepare(c)) return rc;
+    if (c->line_ok != 1) return 0;
+    const size_t rec = size_t(c->nshot) * c->elem_bytes();
+    const size_t sets = c->ckpt > 0 ? 2 : 1;   // the recomputed forward segments interleave with the adjoint steps
+    HRN_CUDA(c, c->d_line_P.alloc(std::max<size_t>(sets * 3 * 9 * c->line_npn * rec, 16)));
+    HRN_CUDA(c, c->d_line_rslot.alloc(std::max<size_t>(size_t(c->nel_rd_e) * 81 * rec, 16)));
+    if (c->line_epoch != c->epoch) {
+        // sources, receivers or history rows on stress equations (none in an ordinary
+        // set-up), and the state rows of the history and the receivers
+        const int first_stress = 3 * c->line_nun;
+        auto stress = [&](const std::vector<int32_t> &eqs) {
+            for (int32_t e : eqs)
+                if (c->line_row[e] >= first_stress) return 1;
+            return 0;
+        };
+        c->line_stress_src = stress(c->h_src_eq) | stress(c->h_eqdis);
+        c->line_stress_hist = stress(c->h_store_eq);
+        auto rows = [&](int n, const DevBuf &eq, DevBuf &out) -> int {
+            HRN_CUDA(c, out.alloc(std::max<size_t>(size_t(n) * 4, 16)));
+            if (n == 0) return 0;
+            k_line_rows<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->d_line_row.as<int32_t>(), eq.as<int32_t>(), out.as<int32_t>());
+            ++c->launches;
+            HRN_CUDA(c, cudaGetLastError());
+            return 0;
+        };
+        if (int rc = rows(c->nstore, c->d_store_eq, c->d_line_store_row)) return rc;
+        if (int rc = rows(c->nrec3, c->d_eqdis, c->d_line_rec_row)) return rc;
+        c->line_epoch = c->epoch;
+    }
+    *ok = 1;
+    return 0;
+}
+
+int line_stage(hrn_ctx *c, const void *args, int stage, int adj, int variant, int first, bool pdl)
+{
+    const int sv = 1 << (variant - 96);
+    return c->precision == HRN_FP64 ? line_stage_f64(c, args, stage, adj, sv, first, pdl) : line_stage_f32(c, args, stage, adj, sv, first, pdl);
+}
+
+}  // namespace hrn

@@ -802,9 +802,17 @@ static int gradient_slots_to_nodes(hrn_ctx *c, double *g_l, double *g_m)
 // ----------------------------------------------------------------------------
 // time loops
 
+// One RK4 step X -> Y.  first: X does not come from the step launched before (the
+// line operator then forms the weighted values of its first stage from X).
+// before_update: an event of other work that reads X; a step that updates X in place
+// waits for it before its last stage.
 template <typename T, int S>
-static void launch_step(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, StageTimer *tm, int lanes, const TileArgs &ta, int adj)
+static void launch_step(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, StageTimer *tm, int lanes, const TileArgs &ta, int adj,
+                        int first, cudaEvent_t before_update = nullptr)
 {
+    // the line operator gathers no state vectors: its last stage updates X in place
+    const bool line = is_line_variant(lanes);
+    if (line) Y = X;
     const size_t vn = size_t(c->neq) * S;
     T *kb = c->d_KB.as<T>();
     a.x1 = X; a.x2 = X + vn; a.x3 = X + 2 * vn;
@@ -817,7 +825,13 @@ static void launch_step(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, StageTimer *tm, 
         T *in = (st == 3) ? mB : mA, *out = (st == 2) ? mB : mA;   // stage s reads set (s%2), writes the other
         a.in_t = in; a.in_m = in + vn; a.in_h = in + 2 * vn;
         a.out_t = out; a.out_m = out + vn; a.out_h = out + 2 * vn;
-        if (is_elem_variant(lanes)) {
+        if (line) {
+            a.in_t = a.out_t = mA;   // replaced by its only reader's successor
+            const bool join = st == 4 && before_update;
+            if (join) cudaStreamWaitEvent(c->stream, before_update, 0);
+            // a stage that follows other work (the step's first, or a join) is launched plainly
+            line_stage(c, &a, st, adj, lanes, first, st > 1 && !join);
+        } else if (is_elem_variant(lanes)) {
             const int b = lanes >= 100 ? 100 : 90;
             elem_stage(c, &a, st, adj, (lanes - b) % 2, 1 << ((lanes - b) / 2), b == 90 ? 1 : 0);
         } else if (is_gt_variant(lanes)) {
@@ -856,16 +870,30 @@ static int autotune_lanes(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, const TileArgs
     float best = 1e30f;
     int pick = 80;
     std::vector<int> cand;
-    if (c->have_pattern) cand.assign(kVariants, kVariants + 10);   // none with a matrix-free operator
-    if (c->have_pattern && gt_ready(c, adj) == 0)
-        // 47 / 87 (pipelined tiles) stay selectable but are not timed here: their many
-        // small bulk copies are limited by the copy engine's rate (about 2x slower)
-        for (int v : {44, 45, 84, 85, 46, 86})
-            if (gt_runs_valid(v, c->nshot, c->elem_bytes())) cand.push_back(v);
-    if (c->op_from_mesh) {
-        if (int rc = elem_ready(c)) return rc;
-        for (int v : {90, 91, 92, 93, 94, 95, 100, 101, 102, 103, 104, 105})
-            if (elem_variant_valid(c, v)) cand.push_back(v);
+    int line = 0;
+    if (c->op_from_mesh)
+        if (int rc = line_ready(c, &line)) return rc;
+    if (line) {
+        // Where the line operator serves the mesh it is 1.4 to 2.2 times as fast as the best
+        // other variant from about 70 thousand equations up; only on the smallest meshes, where
+        // its two launches count, is the row-parallel kernel ahead (8 against 10 us a stage at
+        // 8 thousand equations).  The tables of the others need not be built.
+        if (c->have_pattern) cand = {41, 81};
+        cand.push_back(96);
+        if (c->nshot % 2 == 0) cand.push_back(97);
+        if (c->nshot % 4 == 0 && c->precision == HRN_FP32) cand.push_back(98);
+    } else {
+        if (c->have_pattern) cand.assign(kVariants, kVariants + 10);   // none with a matrix-free operator
+        if (c->have_pattern && gt_ready(c, adj) == 0)
+            // 47 / 87 (pipelined tiles) stay selectable but are not timed here: their many
+            // small bulk copies are limited by the copy engine's rate (about 2x slower)
+            for (int v : {44, 45, 84, 85, 46, 86})
+                if (gt_runs_valid(v, c->nshot, c->elem_bytes())) cand.push_back(v);
+        if (c->op_from_mesh) {
+            if (int rc = elem_ready(c)) return rc;
+            for (int v : {90, 91, 92, 93, 94, 95, 100, 101, 102, 103, 104, 105})
+                if (elem_variant_valid(c, v)) cand.push_back(v);
+        }
     }
     if (cand.empty())
         return set_error(c, HRN_EARG, "no stage variant serves this operator, shot count and precision");
@@ -873,9 +901,9 @@ static int autotune_lanes(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, const TileArgs
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     for (int lanes : cand) {
-        launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj);   // warm-up
+        launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj, 1);   // warm-up
         cudaEventRecord(e0, c->stream);
-        for (int r = 0; r < 3; ++r) launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj);
+        for (int r = 0; r < 3; ++r) launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj, 0);
         cudaEventRecord(e1, c->stream);
         cudaEventSynchronize(e1);
         float ms = 0.f;
@@ -886,6 +914,16 @@ static int autotune_lanes(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, const TileArgs
     cudaEventDestroy(e1);
     HRN_CUDA(c, cudaGetLastError());
     return pick;
+}
+
+// The line variants' tables, or the reason why they cannot run.
+static int line_check(hrn_ctx *c)
+{
+    if (!c->op_from_mesh) return set_error(c, HRN_ESTATE, "the matrix-free variants need an operator assembled from the mesh");
+    int ok = 0;
+    if (int rc = line_ready(c, &ok)) return rc;
+    if (!ok) return set_error(c, HRN_EARG, "the line variants need each node's displacements and stresses numbered in a row");
+    return 0;
 }
 
 static int check_step_error(hrn_ctx *c)
@@ -1014,9 +1052,11 @@ static int forward_t(hrn_ctx *c)
         if (r < 40) return r;
         c->lanes_f = r;
     }
-    if (c->mf_only && !is_elem_variant(c->lanes_f))
-        return set_error(c, HRN_EARG, "the operator is matrix-free: use variants 90-95 / 100-105");
-    if (is_elem_variant(c->lanes_f)) {
+    if (c->mf_only && !is_elem_variant(c->lanes_f) && !is_line_variant(c->lanes_f))
+        return set_error(c, HRN_EARG, "the operator is matrix-free: use variants 90-98 / 100-105");
+    if (is_line_variant(c->lanes_f)) {
+        if (int rc = line_check(c)) return rc;
+    } else if (is_elem_variant(c->lanes_f)) {
         if (!elem_variant_valid(c, c->lanes_f)) return set_error(c, HRN_EARG, "matrix-free variant not available for this shot count and precision");
         if (int rc = elem_ready(c)) return rc;
     } else if (is_gt_variant(c->lanes_f)) {
@@ -1044,7 +1084,8 @@ static int forward_t(hrn_ctx *c)
         const int K = c->ckpt;
         for (int n = 0; n <= c->nstep; ++n) {
             a.srcv = forward_src<T, S>(c, n);
-            T *X = (n & 1) ? X1 : X0, *Y = (n & 1) ? X0 : X1;
+            const bool odd = (n & 1) && !is_line_variant(c->lanes_f);   // line variants step X0 in place
+            T *X = odd ? X1 : X0, *Y = odd ? X0 : X1;
             if (K > 0) {
                 // checkpointed: the state every K steps and the receiver rows of every step
                 if (n % K == 0)
@@ -1052,14 +1093,14 @@ static int forward_t(hrn_ctx *c)
                                                 cudaMemcpyDeviceToDevice, c->stream));
                 if (c->nrec3 > 0) {
                     k_traces<T, S><<<(c->nrec3 * S + 127) / 128, 128, 0, c->stream>>>(
-                        c->nrec3, c->d_eqdis.as<int32_t>(), X + vn, c->d_traces.as<T>() + size_t(n) * c->nrec3 * S);
+                        c->nrec3, (is_line_variant(c->lanes_f) ? c->d_line_rec_row : c->d_eqdis).as<int32_t>(), X + vn, c->d_traces.as<T>() + size_t(n) * c->nrec3 * S);
                     ++c->launches;
                 }
                 a.hist = nullptr;
             } else {
                 a.hist = c->d_hist.as<T>() + size_t(n) * c->nstore * S;
             }
-            launch_step<T, S>(c, a, X, Y, c->timing ? &tm : nullptr, c->lanes_f, ta, 0);
+            launch_step<T, S>(c, a, X, Y, c->timing ? &tm : nullptr, c->lanes_f, ta, 0, n == 0);
         }
         HRN_CUDA(c, cudaGetLastError());
         return 0;
@@ -1085,6 +1126,7 @@ static int forward_t(hrn_ctx *c)
     if (int rc2 = check_step_error(c)) return rc2;
     c->have_forward = true;
     c->have_phist = false;
+    c->fwd_variant = c->lanes_f;
     return 0;
 }
 
@@ -1121,9 +1163,11 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
         if (r < 40) return r;
         c->lanes_a = r;
     }
-    if (c->mf_only && !is_elem_variant(c->lanes_a))
-        return set_error(c, HRN_EARG, "the operator is matrix-free: use variants 90-95 / 100-105");
-    if (is_elem_variant(c->lanes_a)) {
+    if (c->mf_only && !is_elem_variant(c->lanes_a) && !is_line_variant(c->lanes_a))
+        return set_error(c, HRN_EARG, "the operator is matrix-free: use variants 90-98 / 100-105");
+    if (is_line_variant(c->lanes_a)) {
+        if (int rc = line_check(c)) return rc;
+    } else if (is_elem_variant(c->lanes_a)) {
         if (!elem_variant_valid(c, c->lanes_a)) return set_error(c, HRN_EARG, "matrix-free variant not available for this shot count and precision");
         if (int rc = elem_ready(c)) return rc;
     } else if (is_gt_variant(c->lanes_a)) {
@@ -1133,9 +1177,13 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
         if (is_gtp_variant(c->lanes_a))
             if (int rc = gtp_prepare(c, 1)) return rc;
     }
-    if (c->ckpt > 0 && is_gt_variant(c->lanes_f)) {   // the recomputed forward segments
+    if (c->ckpt > 0 && is_line_variant(c->fwd_variant)) {   // the recomputed forward segments
+        if (int rc = line_check(c)) return rc;
+    } else if (c->ckpt > 0 && is_elem_variant(c->fwd_variant)) {
+        if (int rc = elem_ready(c)) return rc;
+    } else if (c->ckpt > 0 && is_gt_variant(c->fwd_variant)) {
         if (int rc = gt_ready(c, 0)) return rc;
-        if (is_gtp_variant(c->lanes_f))
+        if (is_gtp_variant(c->fwd_variant))
             if (int rc = gtp_prepare(c, 0)) return rc;
     }
     cudaEvent_t t0, t1;
@@ -1172,8 +1220,9 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
                 for (int m = k0; m <= m1; ++m) {
                     af.srcv = forward_src<T, S>(c, m);
                     af.hist = c->d_ckseg.as<T>() + size_t(m - k0) * c->nstore * S;
-                    T *Xm = ((m - k0) & 1) ? R1 : R0, *Ym = ((m - k0) & 1) ? R0 : R1;
-                    launch_step<T, S>(c, af, Xm, Ym, c->timing ? &tm : nullptr, c->lanes_f, taf, 0);
+                    const bool odd = ((m - k0) & 1) && !is_line_variant(c->fwd_variant);
+                    T *Xm = odd ? R1 : R0, *Ym = odd ? R0 : R1;
+                    launch_step<T, S>(c, af, Xm, Ym, c->timing ? &tm : nullptr, c->fwd_variant, taf, 0, m == k0);
                 }
             }
             const T *u_n = K > 0 ? c->d_ckseg.as<T>() + size_t(n - k0) * c->nstore * S
@@ -1184,7 +1233,9 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
                     c->d_aslot_eq.as<int32_t>(), rv.map, static_cast<const T *>(rv.hist), c->d_dis.as<double>(),
                     c->d_im.as<double>(), c->d_srcv_a.as<T>(), shot_nstep_ptr(c), rec_mask_ptr(c)); ++c->launches;
             a.hist = keep_p ? c->d_phist.as<T>() + size_t(n) * c->nstore * S : nullptr;
-            T *X = (it & 1) ? X1 : X0, *Y = (it & 1) ? X0 : X1;
+            const bool odd = (it & 1) && !is_line_variant(c->lanes_a);
+            T *X = odd ? X1 : X0, *Y = odd ? X0 : X1;
+            cudaEvent_t reads_x = nullptr;
             if (n <= c->nstep - 1 && c->nel_rd > 0) {
                 // the zero-lag correlation of this step's state runs on the side stream,
                 // next to the step's stages (they read X and write Y, KB, MB)
@@ -1193,18 +1244,20 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
                 k_gradient<T, S><<<gblocks, 128, 0, c->side_stream>>>(c->nel_rd, c->d_rd_store.as<int32_t>(), c->d_rd_elems.as<int32_t>(),
                                                                       c->d_inod.as<int32_t>(), c->d_rd_geom.as<double>(),
                                                                       u_n, X + vn,
-                                                                      c->d_store_eq.as<int32_t>(), gsl, gsm, c->dt, lambda_2mu); ++c->launches;
+                                                                      (is_line_variant(c->lanes_a) ? c->d_line_store_row : c->d_store_eq).as<int32_t>(),
+                                                                      gsl, gsm, c->dt, lambda_2mu); ++c->launches;
                 HRN_CUDA(c, cudaEventRecord(c->ev_join, c->side_stream));
                 forked = true;
+                reads_x = c->ev_join;
             }
-            launch_step<T, S>(c, a, X, Y, c->timing ? &tm : nullptr, c->lanes_a, ta, 1);
+            launch_step<T, S>(c, a, X, Y, c->timing ? &tm : nullptr, c->lanes_a, ta, 1, it == 0, reads_x);
         }
         if (forked) HRN_CUDA(c, cudaStreamWaitEvent(c->stream, c->ev_join, 0));
         if (int rc = gradient_slots_to_nodes(c, gl, gmu)) return rc;
         HRN_CUDA(c, cudaGetLastError());
         return 0;
     };
-    const uint64_t sig[6] = {alloc_generation().load(), c->epoch, uint64_t(c->lanes_a) | (uint64_t(c->lanes_f) << 32),
+    const uint64_t sig[6] = {alloc_generation().load(), c->epoch, uint64_t(c->lanes_a) | (uint64_t(c->fwd_variant) << 32),
                              uint64_t(keep_p != 0), uint64_t(lambda_2mu != 0), uintptr_t(c->stream)};
     const int rc = run_loop(c, c->gadj, sig, body);
     cudaEventRecord(t1, c->stream);
@@ -1315,7 +1368,9 @@ static int time_stage_t(hrn_ctx *c, int adj, int nsteps, double *avg_ms)
     a.srcv = adj ? c->d_srcv_a.as<T>() : forward_src<T, S>(c, 0);
     a.hist = nullptr;
     if (a.nslot > 0 && !a.srcv) return set_error(c, HRN_ESTATE, "no source table: run the time loop first");
-    if (is_elem_variant(lanes)) {
+    if (is_line_variant(lanes)) {
+        if (int rc = line_check(c)) return rc;
+    } else if (is_elem_variant(lanes)) {
         if (int rc = elem_ready(c)) return rc;
     } else if (is_gt_variant(lanes)) {
         if (!gt_runs_valid(lanes, c->nshot, c->elem_bytes())) return set_error(c, HRN_EARG, "variant needs 16-byte records");
@@ -1324,14 +1379,15 @@ static int time_stage_t(hrn_ctx *c, int adj, int nsteps, double *avg_ms)
             if (int rc = gtp_prepare(c, adj)) return rc;
     }
     HRN_CUDA(c, cudaMemsetAsync(X0, 0, 6 * vn * sizeof(T), c->stream));
-    launch_step<T, S>(c, a, X0, X1, nullptr, lanes, ta, adj);   // warm-up
+    launch_step<T, S>(c, a, X0, X1, nullptr, lanes, ta, adj, 1);   // warm-up
     cudaEvent_t e0, e1;
     HRN_CUDA(c, cudaEventCreate(&e0));
     HRN_CUDA(c, cudaEventCreate(&e1));
     cudaEventRecord(e0, c->stream);
     for (int n = 0; n < nsteps; ++n) {
-        T *X = (n & 1) ? X1 : X0, *Y = (n & 1) ? X0 : X1;
-        launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj);
+        const bool odd = (n & 1) && !is_line_variant(lanes);
+        T *X = odd ? X1 : X0, *Y = odd ? X0 : X1;
+        launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj, n == 0);
     }
     cudaEventRecord(e1, c->stream);
     const cudaError_t es = cudaEventSynchronize(e1);

@@ -116,7 +116,7 @@ class Solver:
         self.neq = mesh.neq
 
     def set_operator_mode(self, matrix_free: bool):
-        """True: assemble DIAG_M only and apply C, K, G matrix-free (variants 90-105);
+        """True: assemble DIAG_M only and apply C, K, G matrix-free (variants 90-98 / 100-105);
         call after set_mesh, before the first assemble."""
         self._check(self._L.hrn_set_operator_mode(self.h, int(bool(matrix_free))))
 
@@ -239,7 +239,8 @@ class Solver:
         + 2 for the tiled kernel, + 4 for the compact row tiles with staged
         gathers (40-45, 80-85, 160, 161).  Matrix-free (operator
         assembled from the mesh): 90-95 materialized / 100-105 rebuilt inputs,
-        even = element slots, odd = atomic row sums, with 1, 2 or 4 shots per thread."""
+        even = element slots, odd = atomic row sums, with 1, 2 or 4 shots per thread;
+        96, 97, 98: line operator, up to 1, 2 or 4 shots per thread."""
         self._check(self._L.hrn_set_variant(self.h, int(forward), int(adjoint)))
 
     def variant(self):

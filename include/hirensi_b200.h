@@ -72,7 +72,7 @@ int hrn_set_mesh(hrn_ctx *ctx, int32_t nj, int32_t nel, int32_t neq,
  * matrix_free_only = 0 (default): hrn_assemble builds the CSR of C, K, G as below, and
  * every stage variant is available.  matrix_free_only = 1: hrn_assemble computes only
  * DIAG_M, and C, K, G are applied element by element from the mesh and the nodal
- * material (variants 90-95 / 100-105).  This needs no stored entries, so meshes whose
+ * material (variants 90-98 / 100-105).  This needs no stored entries, so meshes whose
  * CSR would not fit the device (or the 2^31 entry range) can run.  No reference
  * counterpart: the reference always assembles PETSc matrices. */
 int hrn_set_operator_mode(hrn_ctx *ctx, int32_t matrix_free_only);
@@ -287,9 +287,12 @@ int hrn_time_stage(hrn_ctx *ctx, int32_t adjoint, int32_t nsteps, double *avg_st
  * each tile in shared memory with bulk copies, 4 for the kernel over compact
  * row tiles that stages each tile's distinct gathered records in shared
  * memory); lanes in {4, 8, 16}, tiled with 4 or 8.  90-95 / 100-105: the
- * matrix-free element kernels (operator assembled from the mesh).  0 = time all
- * variants on first use and keep the fastest (the default after every new
- * sparsity pattern). */
+ * matrix-free element kernels (operator assembled from the mesh).  96, 97, 98: the
+ * line operator (operator assembled from the mesh) with up to 1, 2, 4 shots per
+ * thread; it needs each node's displacement and stress equations numbered in a row
+ * and PML weights that are constant along the grid lines across them, as on aligned
+ * PML meshes (HRN_EARG otherwise).  0 = time the variants that serve the operator on
+ * first use and keep the fastest (the default after every new sparsity pattern). */
 int hrn_set_variant(hrn_ctx *ctx, int32_t forward, int32_t adjoint);
 int hrn_get_variant(hrn_ctx *ctx, int32_t *forward, int32_t *adjoint);
 
