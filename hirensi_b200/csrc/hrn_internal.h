@@ -195,7 +195,8 @@ struct hrn_ctx {
     hrn::DevBuf d_line_row, d_line_store_row, d_line_rec_row;
     hrn::DevBuf d_line_pnode, d_line_didx, d_line_dcf, d_line_pcoef;
     hrn::DevBuf d_line_unode, d_line_ucoef, d_line_uim, d_line_tidx, d_line_tcf, d_line_ridx;
-    hrn::DevBuf d_line_rpt, d_line_rgeo;
+    hrn::DevBuf d_line_rpt, d_line_rgeo, d_line_runode;
+    hrn::DevBuf d_line_rmat;      // [2][27][nel_rd] scaled lambda, mu of the element points (T)
     hrn::DevBuf d_line_rslot;     // [27][3][nel_rd][S] regular-domain element contributions (T)
     hrn::DevBuf d_line_P;         // [1 or 2 sets][3][9][npn][S] P of this and the next stage, Z (T)
     int fwd_variant = 0;          // variant of the forward whose states the checkpoints hold
@@ -332,6 +333,7 @@ bool elem_variant_valid(const hrn_ctx *c, int variant);
 // line-operator stage: 96, 97, 98 = up to 1, 2, 4 shots per thread (the most that divides
 // the shot count; 4 in FP32 only), so each serves any shot count
 inline bool is_line_variant(int v) { return v >= 96 && v <= 98; }
+bool line_reg_elements(const hrn_ctx *c);
 int line_ready(hrn_ctx *c, int *ok);
 int line_stage(hrn_ctx *c, const void *stage_args, int stage, int adj, int variant, int first, bool pdl);
 int line_stage_f64(hrn_ctx *c, const void *stage_args, int stage, int adj, int sv, int first, bool pdl);

@@ -312,6 +312,9 @@ static int line_tables(hrn_ctx *c)
             ridx[size_t(k - rptr[un_id[u]]) * nun + u] = 3 * c->nel_rd_e * q + e;
         }
     for (auto &p : rpt) p.y = unidx[p.x];
+    std::vector<int32_t> runode(rpt.size(), -1);   // by point, then element
+    for (int e = 0; e < c->nel_rd_e; ++e)
+        for (int q = 0; q < 27; ++q) runode[size_t(q) * c->nel_rd_e + e] = rpt[size_t(e) * 27 + q].y;
     std::vector<int32_t> zidx(pidx);   // records of Z: PML nodes whose displacements are free
     for (int j = 0; j < nj; ++j)
         if (ubase[j] < 0) zidx[j] = -1;
@@ -325,6 +328,7 @@ static int line_tables(hrn_ctx *c)
     if (int rc = put(c->d_line_unode, unode.data(), unode.size() * 16)) return rc;
     if (int rc = put(c->d_line_ridx, ridx.data(), ridx.size() * 4)) return rc;
     if (int rc = put(c->d_line_rpt, rpt.data(), rpt.size() * 8)) return rc;
+    if (int rc = put(c->d_line_runode, runode.data(), runode.size() * 4)) return rc;
     if (int rc = put(c->d_line_row, row.data(), row.size() * 4)) return rc;
     if (int rc = put(d_pn, pn_id.data(), pn_id.size() * 4)) return rc;
     if (int rc = put(d_pe, pn_eq.data(), pn_eq.size() * 4)) return rc;
@@ -399,6 +403,17 @@ static int line_prepare(hrn_ctx *c)
     return 0;
 }
 
+// Whether the regular-domain elements take the kernel that keeps an element in one
+// thread's registers: FP32 (in FP64 an element does not fit) boxes, and enough of them to
+// hide its longer chain and the extra launch.  Elements x shots, us a stage with the
+// thread-per-point blocks / with the register kernel: 8 thousand 17.2 / 23.1, 16 thousand
+// 29.5 / 34.4, 28 thousand 40.0 / 41.4, 61 thousand 151 / 125, 256 thousand 253 / 197.
+constexpr int64_t kLineRegElements = 50000;
+bool line_reg_elements(const hrn_ctx *c)
+{
+    return c->precision == HRN_FP32 && c->line_box && int64_t(c->nel_rd_e) * c->nshot >= kLineRegElements;
+}
+
 // Tables and buffers for the current shots; *ok = 0 when the mesh needs another variant.
 int line_ready(hrn_ctx *c, int *ok)
 {
@@ -409,6 +424,7 @@ int line_ready(hrn_ctx *c, int *ok)
     const size_t rec = size_t(c->nshot) * c->elem_bytes();
     const size_t sets = c->ckpt > 0 ? 2 : 1;   // the recomputed forward segments interleave with the adjoint steps
     HRN_CUDA(c, c->d_line_P.alloc(std::max<size_t>(sets * 3 * 9 * c->line_npn * rec, 16)));
+    if (line_reg_elements(c)) HRN_CUDA(c, c->d_line_rmat.alloc(size_t(c->nel_rd_e) * 54 * c->elem_bytes()));
     HRN_CUDA(c, c->d_line_rslot.alloc(std::max<size_t>(size_t(c->nel_rd_e) * 81 * rec, 16)));
     if (c->line_epoch != c->epoch) {
         // sources, receivers or history rows on stress equations (none in an ordinary

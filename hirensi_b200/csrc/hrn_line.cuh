@@ -43,10 +43,10 @@
 // bytes per entry besides; here a node gathers about 21 records of three rows for
 // all of its nine rows, and streams as many small entries.  Microseconds a stage
 // (forward), best other variant -> here:
-//     16 x 16 x 8 + PML 3, FP64, 4 shots   68.6 -> 31.8      FP32, 4 shots   37.0 -> 17.0
+//     16 x 16 x 8 + PML 3, FP64, 4 shots   68.6 -> 29.9      FP32, 4 shots   37.0 -> 17.0
 //     the same, FP64, 1 shot               30.7 -> 13.1
 //     11 x 7 x 5 + PML 2, FP64, 3 shots    19.0 -> 12.3
-//     40 x 40 x 20 + PML 3, FP32, 8 shots   372 -> 253
+//     40 x 40 x 20 + PML 3, FP32, 8 shots   372 -> 197
 #pragma once
 
 #include <cuda_runtime.h>
@@ -92,6 +92,8 @@ struct LineArgs {
     const double *__restrict__ rgeo;     // boxes: [nrd][4] DJI_y / DJI_x, DJI_z / DJI_x, detJ DJI_x^2, 0; else
                                          // [nrd * 27][10] DJI and w*detJ
     const double *__restrict__ lam, *__restrict__ mu;
+    const int32_t *__restrict__ runode;  // [27][nrd] displacement node of the element's point (-1: constrained)
+    T *rlam, *rmu;                       // [27][nrd] lambda, mu times w detJ DJI_x^2 of the point
     // written by the launches of a loop
     T *x1, *x2, *x3, *k1, *k2, *k3;      // [3][nun][S], then [6][npn][S]
     T *kt;                               // [3][nun][S] K's input at the regular-domain nodes
@@ -276,8 +278,10 @@ template <int S, int SV>
 constexpr int line_elems() { return line_threads<S, SV>() / (27 * (S / SV)); }
 template <int S, int SV>
 constexpr int line_nodes() { return line_threads<S, SV>() / (S / SV); }
-template <typename T, int S, int SV>
-constexpr int line_blocks() { return (SV * sizeof(T) > 8 ? 384 : 640) / line_threads<S, SV>(); }
+// Resident blocks the register limits leave: k_line_a needs up to 168 registers a thread
+// with 16 bytes of shots and 96 with 8; k_line_b does better with 128 in the first case.
+template <typename T, int S, int SV, int B>
+constexpr int line_blocks() { return (SV * sizeof(T) > 8 ? (B ? 512 : 384) : 640) / line_threads<S, SV>(); }
 template <typename T, int S, int SV, int BOX>
 constexpr size_t line_smem() { return size_t(line_elems<S, SV>()) * 27 * (3 + (BOX ? 6 : 9)) * S * sizeof(T); }
 
@@ -441,6 +445,93 @@ __device__ __forceinline__ void line_rd_elements(const LineArgs<T> &L, const T *
     for (int c = 0; c < 3; ++c) stv<T, SV>(o + size_t(c) * L.nrd * S, y[c]);
 }
 
+// The same for large grids in FP32, with one thread per (box element, shot): the 81
+// displacements and the 81 sums of an element live in its thread's registers (254 of
+// them).  With a thread per point the kernel is bound by shared memory (39 reads and 9
+// writes a point and shot); here nothing passes through it: 88 -> 45 us a stage for 32000
+// elements and 8 shots, 113 MB.
+template <typename T, int S>
+__global__ void __launch_bounds__(64, 4) k_line_r(const LineArgs<T> L, const T *ut)
+{
+    dep_trigger();
+    const int64_t tid = blockIdx.x * int64_t(64) + threadIdx.x;
+    const int64_t e64 = tid / S;
+    if (e64 >= L.nrd) return;
+    const int e = int(e64), s = int(tid % S);
+    const size_t nrd = size_t(L.nrd);
+    const T r[3] = {T(1), T(__ldg(L.rgeo + size_t(e) * 4)), T(__ldg(L.rgeo + size_t(e) * 4 + 1))};
+    T u[3][27], y[3][27];
+    int id[27];
+#pragma unroll
+    for (int q = 0; q < 27; ++q) id[q] = __ldg(L.runode + q * nrd + e);
+    dep_wait();
+#pragma unroll
+    for (int q = 0; q < 27; ++q)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            T v[1];
+            ldw_if<T, 1>(id[q] >= 0, ut + (size_t(c) * L.nun + uint32_t(id[q])) * S + s, v);
+            u[c][q] = v[0];
+            y[c][q] = T(0);
+        }
+    constexpr int str[3] = {1, 3, 9};
+    constexpr T D[3][3] = {{T(-1.5), T(2), T(-0.5)}, {T(-0.5), T(0), T(0.5)}, {T(0.5), T(-2), T(1.5)}};
+#pragma unroll
+    for (int q = 0; q < 27; ++q) {
+        const int qm[3] = {q % 3, (q / 3) % 3, q / 9};
+        T g[3][3];   // d u_c / d x_m
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int b = q - qm[m] * str[m];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                T v = D[qm[m]][0] * u[c][b];
+                if (qm[m] != 1) v = fmaT(D[qm[m]][1], u[c][b + str[m]], v);
+                v = fmaT(D[qm[m]][2], u[c][b + 2 * str[m]], v);
+                g[c][m] = m > 0 ? v * r[m] : v;
+            }
+        }
+        const T lam = L.rlam[q * nrd + e], mu = L.rmu[q * nrd + e], m2 = T(2) * mu;
+        const T tr = lam * (g[0][0] + g[1][1] + g[2][2]);
+        T f[3][3];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            f[c][c] = fmaT(m2, g[c][c], tr);
+#pragma unroll
+            for (int m = c + 1; m < 3; ++m) f[c][m] = f[m][c] = mu * (g[c][m] + g[m][c]);
+        }
+#pragma unroll
+        for (int m = 0; m < 3; ++m) {
+            const int b = q - qm[m] * str[m];
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+                const T v = m > 0 ? f[c][m] * r[m] : f[c][m];
+                y[c][b] = fmaT(D[qm[m]][0], v, y[c][b]);
+                if (qm[m] != 1) y[c][b + str[m]] = fmaT(D[qm[m]][1], v, y[c][b + str[m]]);
+                y[c][b + 2 * str[m]] = fmaT(D[qm[m]][2], v, y[c][b + 2 * str[m]]);
+            }
+        }
+    }
+    T *o = L.rslot + size_t(e) * S + s;
+#pragma unroll
+    for (int q = 0; q < 27; ++q)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) o[size_t(3 * q + c) * nrd * S] = y[c][q];
+}
+// Its material: lambda, mu of the points times w detJ DJI_x^2, formed in FP64.
+template <typename T>
+__global__ void __launch_bounds__(256) k_line_material(const LineArgs<T> L)
+{
+    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (t >= int64_t(27) * L.nrd) return;
+    const int q = int(t / L.nrd), e = int(t % L.nrd);
+    const double third = 1.0 / 3.0, mid = 4.0 / 3.0;   // GLL weights
+    const double f = __ldg(L.rgeo + size_t(e) * 4 + 2) * (q % 3 == 1 ? mid : third) * (q / 3 % 3 == 1 ? mid : third) * (q / 9 == 1 ? mid : third);
+    const int node = __ldg(L.rpt + size_t(e) * 27 + q).x;
+    L.rlam[t] = T(f * __ldg(L.lam + node));
+    L.rmu[t] = T(f * __ldg(L.mu + node));
+}
+
 // Stress rows of one PML node and the P of its next inputs.
 template <typename T, int S, int SV, int stage, int ADJ>
 __device__ __forceinline__ void line_stress_rows(const LineArgs<T> &L, int block)
@@ -573,7 +664,7 @@ __device__ __forceinline__ void line_stress_rows(const LineArgs<T> &L, int block
 }
 
 template <typename T, int S, int SV, int stage, int ADJ, int BOX>
-__global__ void __launch_bounds__(line_threads<S, SV>(), line_blocks<T, S, SV>()) k_line_a(const LineArgs<T> L, int nb_stress)
+__global__ void __launch_bounds__(line_threads<S, SV>(), line_blocks<T, S, SV, 0>()) k_line_a(const LineArgs<T> L, int nb_stress)
 {
     extern __shared__ __align__(16) unsigned char line_sm[];
     dep_trigger();
@@ -635,7 +726,7 @@ __global__ void __launch_bounds__(256) k_line_z0(const LineArgs<T> L)
 
 // Displacement rows of one node; nodes of the PML first.
 template <typename T, int S, int SV, int stage, int ADJ>
-__global__ void __launch_bounds__(line_threads<S, SV>(), line_blocks<T, S, SV>()) k_line_b(const LineArgs<T> L)
+__global__ void __launch_bounds__(line_threads<S, SV>(), line_blocks<T, S, SV, 1>()) k_line_b(const LineArgs<T> L)
 {
     constexpr int TP = S / SV, N = 4;   // records in flight
     dep_trigger();
@@ -784,7 +875,20 @@ static void line_launch(hrn_ctx *c, LineArgs<T> &L, int first, bool pdl)
     }
     L.P = buf + ((STAGE - 1) & 1) * psz;
     L.Pn = buf + (STAGE & 1) * psz;
-    const int nb_s = (L.npn + NPB - 1) / NPB, nb_r = (L.nrd + EPB - 1) / EPB;
+    const int nb_s = (L.npn + NPB - 1) / NPB;
+    int nb_r = (L.nrd + EPB - 1) / EPB;
+    if constexpr (sizeof(T) == 4) {
+        if (line_reg_elements(c)) {
+            if (STAGE == 1 && first) {
+                k_line_material<T><<<unsigned((int64_t(27) * L.nrd + 255) / 256), 256, 0, c->stream>>>(L);
+                ++c->launches;
+            }
+            line_start(k_line_r<T, S>, int((int64_t(L.nrd) * S + 63) / 64), 64, 0, c->stream, pdl, L, static_cast<const T *>(STAGE == 1 ? L.x2 : L.kt));
+            ++c->launches;
+            pdl = true;
+            nb_r = 0;
+        }
+    }
     if (nb_s + nb_r > 0) {
         static_assert(line_smem<T, S, SV, 0>() <= 48 * 1024, "k_line_a exceeds the default shared memory of a CTA");
         if (c->line_box)
@@ -820,6 +924,9 @@ static LineArgs<T> line_args(hrn_ctx *c, const StageArgs<T> &a, int set)
     L.uim = c->d_line_uim.as<double>();
     L.rpt = c->d_line_rpt.as<int2>();
     L.rgeo = c->d_line_rgeo.as<double>();
+    L.runode = c->d_line_runode.as<int32_t>();
+    L.rlam = c->d_line_rmat.as<T>();
+    L.rmu = L.rlam + size_t(27) * c->nel_rd_e;
     L.lam = c->d_lam.as<double>();
     L.mu = c->d_mu.as<double>();
     L.x1 = const_cast<T *>(a.x1);

@@ -188,3 +188,27 @@ def test_variant_survives_another_shot_count(gpu_lib):
         s.set_variant(41, 41)
         s.forward()
         assert rel_l2(odd, s.traces()) < 1e-11
+
+
+@pytest.mark.parametrize("nshot,variant", [(8, 98), (7, 96)])
+def test_register_elements_of_large_fp32_grids(gpu_lib, nshot, variant):
+    """Enough elements and shots for the kernel that keeps an element in registers."""
+    from hirensi_b200.configs import inversion_config
+    from hirensi_b200.solver import Solver
+    p = inversion_config(nstep=12, nx=21, ny=20, nz=18, npml=1, shots=tuple((2.5 * k - 10.0, 5.0) for k in range(nshot)),
+                         receivers=(-10.0, 0.0, 10.0), fr=900.0)
+    dis = 1e-6 * np.random.default_rng(2).standard_normal((nshot, len(p.eqdis), p.nstep + 1))
+    out = {}
+    for prec, v in (("fp32", variant), ("fp64", 41)):
+        with Solver(prec) as s:
+            s.set_mesh(p.mesh, RHO)
+            s.assemble(p.lam_true, p.mu_true)
+            s.set_history(p.mesh.store_eq)
+            s.set_shots(p.nstep, p.dt, p.src_eq, p.src_b, p.ftab)
+            s.set_receivers(p.eqdis, p.eqdis_map)
+            s.set_variant(v, v)
+            s.forward()
+            s.misfit(dis)
+            out[prec] = (s.history(nshot - 1), *s.adjoint_gradient(dis))
+    for a, b, bar in zip(out["fp32"], out["fp64"], (1e-4, 1e-3, 1e-3)):
+        assert rel_l2(a, b) < bar
