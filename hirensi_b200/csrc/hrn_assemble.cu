@@ -46,6 +46,8 @@ struct AsmArgs {
     int nel;
     const int32_t *inod, *id;
     const double *xyz, *geom, *lam, *mu, *rho, *pml;
+    const double *pmlf;         // [nj][12] stretching factors of every node (k_asm_pml), -1 in [0] past the top
+    const double *pmla;         // [nj] the factor a
     // values mode
     const int32_t *rowptr;
     const uint32_t *colx;
@@ -175,12 +177,18 @@ __global__ void k_asm_rd_k(AsmArgs A)
 
 // One thread per (element, local node): diagonal mass of the RD (ELEMENT_M_3D, flag 201),
 // and for PML elements the diagonal blocks EM_a..d (flags 202-205), EN_a..d (301-304).
+// One thread a factor and DOF for the PML's (kDiagParts: the mass, then 9 DOF of b, c, d),
+// each with its own search in the pattern: 27 searches in sequence took 80 us a colour.
+constexpr int kDiagParts = 1 + 3 * 9;
 __global__ void k_asm_diag(AsmArgs A, int pml)
 {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= A.nel * 27) return;
-    const int I = t % 27;
+    const int64_t tt = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    const int parts = pml ? (A.no_csr ? 1 : kDiagParts) : 1;
+    const int64_t t = tt / parts;
+    if (t >= int64_t(A.nel) * 27) return;
+    const int I = int(t % 27);
     const int e = A.elems[t / 27];
+    const int k = int(tt % parts), part = k == 0 ? 0 : 1 + (k - 1) / 9, dof = k == 0 ? 0 : (k - 1) % 9;
     const int node = A.inod[size_t(e) * 27 + I];
     const int q = 9 * a_ijk[I][2] + 3 * a_ijk[I][1] + a_ijk[I][0];
     const double fac0 = A.geom[(size_t(e) * 27 + q) * 10 + 9];
@@ -193,26 +201,46 @@ __global__ void k_asm_diag(AsmArgs A, int pml)
             if (idn[cc] >= 0) A.diag_m[idn[cc]] = add(A.diag_m[idn[cc]], v);
         return;
     }
-    double ab[10];
-    const double *x = A.xyz + size_t(node) * 3;
-    if (!pml_ab(x, A.pml, ab)) { atomicExch(A.err, 4); return; }
+    const double *F = A.pmlf + size_t(node) * 12;
+    if (F[0] < 0.0) { atomicExch(A.err, 4); return; }
     // EM_f (u) and EN_f (s) diagonal values for f = a, b, c, d
-    for (int f = 0; f < 4; ++f) {
-        const double fm = mul(rho, ab[6 + f]);
-        const double vu = mul(mul(fm, 1.0), fac0);
-        const double vs1 = mul(mul(ab[6 + f], 1.0), fac0);
-        const double vs2 = mul(mul(mul(2.0, ab[6 + f]), 1.0), fac0);
-        if (f == 0) {
-            if (A.discover) continue;
-            for (int cc = 0; cc < 3; ++cc)
-                if (idn[cc] >= 0) A.diag_m[idn[cc]] = add(A.diag_m[idn[cc]], vu);
-            for (int cc = 0; cc < 6; ++cc)
-                if (idn[3 + cc] >= 0) A.diag_m[idn[3 + cc]] = add(A.diag_m[idn[3 + cc]], cc < 3 ? vs1 : vs2);
-            continue;
-        }
-        for (int cc = 0; cc < 3; ++cc) put(A, idn[cc], idn[cc], f - 1, vu);
-        for (int cc = 0; cc < 6; ++cc) put(A, idn[3 + cc], idn[3 + cc], f - 1, cc < 3 ? vs1 : vs2);
+    const double f = part == 0 ? A.pmla[node] : F[8 + part];
+    const double vu = mul(mul(mul(rho, f), 1.0), fac0);
+    const double vs1 = mul(mul(f, 1.0), fac0);
+    const double vs2 = mul(mul(mul(2.0, f), 1.0), fac0);
+    if (part == 0) {
+        if (A.discover) return;
+        for (int cc = 0; cc < 3; ++cc)
+            if (idn[cc] >= 0) A.diag_m[idn[cc]] = add(A.diag_m[idn[cc]], vu);
+        for (int cc = 0; cc < 6; ++cc)
+            if (idn[3 + cc] >= 0) A.diag_m[idn[3 + cc]] = add(A.diag_m[idn[3 + cc]], cc < 3 ? vs1 : vs2);
+        return;
     }
+    const int cc = dof;
+    put(A, idn[cc], idn[cc], part - 1, cc < 3 ? vu : (cc < 6 ? vs1 : vs2));
+}
+
+// Stretching factors of every node: F1, F2, F3 of the kinds e, p, w, then b, c, d; a first
+// entry of -1 marks a node past the top face.  The element kernels take them from here: each
+// EA entry used to evaluate the whole profile again (three divisions for a value that most
+// entries then multiply by a zero derivative).
+__global__ void k_asm_pml(int nj, const double *__restrict__ xyz, const double *__restrict__ pml, double *__restrict__ out,
+                          double *__restrict__ a)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= nj) return;
+    double ab[10], *o = out + size_t(j) * 12;
+    if (!pml_ab(xyz + size_t(j) * 3, pml, ab)) {
+        o[0] = -1.0;
+        return;
+    }
+    o[0] = mul(ab[0], ab[1]); o[1] = mul(ab[0], ab[2]); o[2] = mul(ab[1], ab[2]);
+    o[3] = add(mul(ab[0], ab[4]), mul(ab[1], ab[3]));
+    o[4] = add(mul(ab[0], ab[5]), mul(ab[2], ab[3]));
+    o[5] = add(mul(ab[1], ab[5]), mul(ab[2], ab[4]));
+    o[6] = mul(ab[3], ab[4]); o[7] = mul(ab[3], ab[5]); o[8] = mul(ab[4], ab[5]);
+    o[9] = ab[7]; o[10] = ab[8]; o[11] = ab[9];
+    a[j] = ab[6];
 }
 
 // One thread per (element, EA pair (I, J), c, d, kind e/p/w): the upper EA value goes
@@ -234,19 +262,17 @@ __global__ void k_asm_ea(AsmArgs A)
     const int q = 9 * a_ijk[J][2] + 3 * a_ijk[J][1] + a_ijk[J][0];
     const double *g = A.geom + (size_t(e) * 27 + q) * 10;
     const int nq = nd[J];
-    double ab[10];
-    if (!pml_ab(A.xyz + size_t(nq) * 3, A.pml, ab)) { atomicExch(A.err, 4); return; }
-    double F1, F2, F3;
-    if (kind == 0) { F1 = mul(ab[0], ab[1]); F2 = mul(ab[0], ab[2]); F3 = mul(ab[1], ab[2]); }
-    else if (kind == 1) {
-        F1 = add(mul(ab[0], ab[4]), mul(ab[1], ab[3]));
-        F2 = add(mul(ab[0], ab[5]), mul(ab[2], ab[3]));
-        F3 = add(mul(ab[1], ab[5]), mul(ab[2], ab[4]));
-    } else { F1 = mul(ab[3], ab[4]); F2 = mul(ab[3], ab[5]); F3 = mul(ab[4], ab[5]); }
     double fi[3];
     dfx_row(I, q, g, fi);
     const double h1 = mul(fi[0], 1.0), h2 = mul(fi[1], 1.0), h3 = mul(fi[2], 1.0), h4 = (I == J) ? 1.0 : 0.0;
+    // entries of a direction without a derivative are zero (I and J off its line)
+    const double hd = (d == 3 ? (c == 0 ? h2 : h1) : d == 4 ? (c == 0 ? h3 : h1) : d == 5 ? (c == 1 ? h3 : h2)
+                                                                                          : (c == 0 ? h1 : c == 1 ? h2 : h3));
+    const double *F = A.pmlf + size_t(nq) * 12;
+    if (F[0] < 0.0) { atomicExch(A.err, 4); return; }
     const double zl = A.lam[nq], zm = A.mu[nq];
+    if (hd == 0.0 && isfinite(zl) && isfinite(zm)) return;   // 0 times a non-finite modulus is not
+    const double F1 = F[3 * kind], F2 = F[3 * kind + 1], F3 = F[3 * kind + 2];
     double vals[2];
     for (int lower = 0; lower < 2; ++lower) {
         const double f7 = lower ? add(zl, mul(2.0, zm)) : 1.0;
@@ -385,7 +411,7 @@ static int run_group(hrn_ctx *c, AsmArgs A, int g, int off, int n)
     A.elems = c->d_el_color_list.as<int32_t>() + c->color_off[g] + off;
     A.nel = n;
     const bool pml = (g % 2) == 1;
-    k_asm_diag<<<(n * 27 + th - 1) / th, th, 0, c->stream>>>(A, pml ? 1 : 0); ++c->launches;
+    k_asm_diag<<<unsigned((int64_t(n) * 27 * (pml ? kDiagParts : 1) + th - 1) / th), th, 0, c->stream>>>(A, pml ? 1 : 0); ++c->launches;
     if (!pml) {
         const int64_t tot = int64_t(n) * 513 * 9;
         k_asm_rd_k<<<unsigned((tot + th - 1) / th), th, 0, c->stream>>>(A); ++c->launches;
@@ -453,6 +479,15 @@ int assemble_device(hrn_ctx *c, bool discover_pattern)
     A.mu = c->d_mu.as<double>();
     A.rho = c->d_rho.as<double>();
     A.pml = c->d_pml.as<double>();
+    if (!c->have_asm_pml) {
+        HRN_CUDA(c, c->d_asm_pmlf.alloc(size_t(c->nj) * 13 * 8));
+        k_asm_pml<<<(c->nj + 255) / 256, 256, 0, c->stream>>>(c->nj, A.xyz, A.pml, c->d_asm_pmlf.as<double>(),
+                                                              c->d_asm_pmlf.as<double>() + size_t(c->nj) * 12); ++c->launches;
+        HRN_CUDA(c, cudaGetLastError());
+        c->have_asm_pml = true;
+    }
+    A.pmlf = c->d_asm_pmlf.as<double>();
+    A.pmla = A.pmlf + size_t(c->nj) * 12;
     A.err = c->d_asm_err.as<int>();
     HRN_CUDA(c, cudaMemsetAsync(c->d_asm_err.p, 0, 16, c->stream));
     if (c->mf_only) return assemble_mass_only(c, A);

@@ -152,6 +152,7 @@ struct hrn_ctx {
     std::vector<double> h_xyz, h_rho, h_pml;
     std::vector<int32_t> h_inod, h_mtel, h_id;
     hrn::DevBuf d_xyz, d_inod, d_id, d_rho, d_pml;
+    bool rd_box = false;          // every regular-domain element is an axis-aligned box
     hrn::DevBuf d_rd_elems;       // [nel_rd] element ids of the regular domain
     hrn::DevBuf d_rd_geom;        // [nel_rd][27][10] DJI (9) and w*detJ per GLL point (FP64)
     hrn::DevBuf d_rd_store;       // [nel_rd][27] history node index (store index / 3)
@@ -164,6 +165,8 @@ struct hrn_ctx {
     std::vector<int> color_off;   // [ncolor + 1]
     hrn::DevBuf d_lam, d_mu;      // nodal material (FP64)
     hrn::DevBuf d_touched;        // pattern discovery flags
+    hrn::DevBuf d_asm_pmlf;       // [nj][12] stretching factors, then [nj] the factor a (FP64)
+    bool have_asm_pml = false;
     hrn::DevBuf d_asm_err;        // device error flag of the assembly kernels
     hrn::DevBuf d_face_b;         // [neq] face-traction force vector B (FP64)
     bool have_face_b = false;
@@ -186,7 +189,6 @@ struct hrn_ctx {
     // line-operator stage (variants 96-98): tables of the mesh, see hrn_line.cuh
     bool have_line = false;
     int line_ok = 0;              // 1: the mesh suits it, -1: it does not
-    int line_box = 0;             // every regular-domain element is an axis-aligned box
     int line_npn = 0, line_nup = 0, line_nun = 0;   // PML nodes; displacement nodes in the PML, all
     int line_wd = 0, line_wt = 0;
     int line_stress_src = 0, line_stress_hist = 0;

@@ -25,8 +25,6 @@ constexpr int kLineCoefPlanes = 15;
 constexpr double kLineDrop = 16 * 2.2204460492503131e-16;
 // PML weights that differ by less along a line are the same value with rounding.
 constexpr double kWeightTol = 1e-13;
-// An element counts as an axis-aligned box when its DJI and detJ vary by less than this.
-constexpr double kBoxTol = 1e-13;
 
 __device__ __forceinline__ double gll_d(int a, int b)   // l_b'(xi_a)
 {
@@ -157,25 +155,6 @@ __global__ void k_line_rows(int n, const int32_t *__restrict__ row, const int32_
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) out[i] = row[eq[i]];
-}
-
-// Axis-aligned boxes: DJI diagonal and the same, like detJ, at all 27 points.
-__global__ void k_line_box(int nrd, const double *__restrict__ geom, int *__restrict__ bad)
-{
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nrd * 27) return;
-    const double *g = geom + size_t(t) * 10, *c = geom + (size_t(t / 27) * 27 + 13) * 10;
-    const int q = t % 27;
-    auto w = [](int a) { return a == 1 ? 4.0 / 3.0 : 1.0 / 3.0; };
-    const double wq = w(q % 3) * w((q / 3) % 3) * w(q / 9), wc = 64.0 / 27.0;
-    bool ok = fabs(g[9] * wc - c[9] * wq) <= kBoxTol * c[9] * wq;
-    double dmin = fmin(fabs(c[0]), fmin(fabs(c[4]), fabs(c[8])));
-    for (int m = 0; m < 3; ++m)
-        for (int k = 0; k < 3; ++k) {
-            const double v = g[3 * m + k];
-            ok = ok && (m == k ? fabs(v - c[4 * m]) <= kBoxTol * fabs(c[4 * m]) : fabs(v) <= kBoxTol * dmin);
-        }
-    if (!ok) atomicExch(bad, 1);
 }
 
 __global__ void k_line_rgeo(int64_t n, int box, const double *__restrict__ geom, double *__restrict__ out)
@@ -370,20 +349,15 @@ static int line_tables(hrn_ctx *c)
     ++c->launches;
     HRN_CUDA(c, cudaGetLastError());
     const double *rg = c->d_el_geom.as<double>() + size_t(c->nel_pml_e) * 270;
-    if (c->nel_rd_e > 0) {
-        k_line_box<<<(c->nel_rd_e * 27 + 255) / 256, 256, 0, c->stream>>>(c->nel_rd_e, rg, bad.as<int>() + 1);
-        ++c->launches;
-        HRN_CUDA(c, cudaGetLastError());
-    }
-    int flags[2];
-    HRN_CUDA(c, cudaMemcpyAsync(flags, bad.p, 8, cudaMemcpyDeviceToHost, c->stream));
+    int flag = 0;
+    HRN_CUDA(c, cudaMemcpyAsync(&flag, bad.p, 4, cudaMemcpyDeviceToHost, c->stream));
     HRN_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (flags[0]) return 0;   // too many nodes on the lines of one, or weights that vary along a line
-    c->line_box = flags[1] ? 0 : 1;
-    const int64_t ng = int64_t(c->nel_rd_e) * (c->line_box ? 4 : 270);
+    if (flag) return 0;   // too many nodes on the lines of one, or weights that vary along a line
+    const int box = c->rd_box ? 1 : 0;
+    const int64_t ng = int64_t(c->nel_rd_e) * (box ? 4 : 270);
     HRN_CUDA(c, c->d_line_rgeo.alloc(std::max<size_t>(size_t(ng), 1) * 8));
     if (ng > 0) {
-        k_line_rgeo<<<unsigned((ng + 255) / 256), 256, 0, c->stream>>>(ng, c->line_box, rg, c->d_line_rgeo.as<double>());
+        k_line_rgeo<<<unsigned((ng + 255) / 256), 256, 0, c->stream>>>(ng, box, rg, c->d_line_rgeo.as<double>());
         ++c->launches;
         HRN_CUDA(c, cudaGetLastError());
     }
@@ -411,7 +385,7 @@ static int line_prepare(hrn_ctx *c)
 constexpr int64_t kLineRegElements = 50000;
 bool line_reg_elements(const hrn_ctx *c)
 {
-    return c->precision == HRN_FP32 && c->line_box && int64_t(c->nel_rd_e) * c->nshot >= kLineRegElements;
+    return c->precision == HRN_FP32 && c->rd_box && int64_t(c->nel_rd_e) * c->nshot >= kLineRegElements;
 }
 
 // Tables and buffers for the current shots; *ok = 0 when the mesh needs another variant.

@@ -891,7 +891,7 @@ static void line_launch(hrn_ctx *c, LineArgs<T> &L, int first, bool pdl)
     }
     if (nb_s + nb_r > 0) {
         static_assert(line_smem<T, S, SV, 0>() <= 48 * 1024, "k_line_a exceeds the default shared memory of a CTA");
-        if (c->line_box)
+        if (c->rd_box)
             line_start(k_line_a<T, S, SV, STAGE, ADJ, 1>, nb_s + nb_r, NT, line_smem<T, S, SV, 1>(), c->stream, pdl, L, nb_s);
         else
             line_start(k_line_a<T, S, SV, STAGE, ADJ, 0>, nb_s + nb_r, NT, line_smem<T, S, SV, 0>(), c->stream, pdl, L, nb_s);
