@@ -64,6 +64,17 @@ struct DevBuf {
     template <typename T> T *as() const { return static_cast<T *>(p); }
 };
 
+// Owning page-locked host buffer that kernels write scalars to (read after a synchronisation).
+struct HostBuf {
+    void *p = nullptr;
+    HostBuf() = default;
+    HostBuf(const HostBuf &) = delete;
+    HostBuf &operator=(const HostBuf &) = delete;
+    ~HostBuf() { if (p) cudaFreeHost(p); }
+    cudaError_t alloc(size_t n) { return p ? cudaSuccess : cudaHostAlloc(&p, n, cudaHostAllocPortable | cudaHostAllocMapped); }
+    template <typename T> T *as() const { return static_cast<T *>(p); }
+};
+
 constexpr int kTagBits = 30;
 constexpr int kTileEntries = 4096;     // entries per tile of the tiled stage kernel
 constexpr size_t kBulkPad = 64;        // bytes past the end of bulk-copied arrays
@@ -258,12 +269,12 @@ struct hrn_ctx {
     bool have_data = false;       // measured data resident on the device
 
     // ---- inversion (model update)
-    hrn::DevBuf d_red;            // reduction partials
+    hrn::DevBuf d_red;            // reduction partials and the count of finished blocks
+    hrn::HostBuf h_red;           // [4] scalars that the reductions return
     hrn::DevBuf d_tv_part;        // per-block partial sums of the TV regularization
     int lbfgs_m = 0;
-    hrn::DevBuf d_lbfgs;          // [4][M][nj] Ys_l, Ys_m, Ss_l, Ss_m, then 6 scratch vectors [nj]
+    hrn::DevBuf d_lbfgs;          // [4][M][nj] Ys_l, Ys_m, Ss_l, Ss_m, q_l, q_m [nj], then rho[M], alpha[M], H0 and partials
     hrn::DevBuf d_restrict;       // [nj] restriction to the regular domain (1 / 0)
-    std::vector<double> lbfgs_rho, lbfgs_alpha;
 
     // ---- CUDA graphs of the time loops (on unless disabled or timing per launch)
     bool graphs = true;

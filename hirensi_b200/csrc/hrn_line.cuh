@@ -57,6 +57,7 @@
 #include <utility>
 
 #include "hrn_internal.h"
+#include "hrn_pdl.cuh"
 #include "hrn_stage.cuh"
 
 namespace hrn {
@@ -121,11 +122,6 @@ __device__ __forceinline__ void gll_dcol(int b, T &d0, T &d1, T &d2)
     d1 = b == 0 ? T(-0.5) : (b == 1 ? T(0.0) : T(0.5));
     d2 = b == 0 ? T(0.5) : (b == 1 ? T(-2.0) : T(1.5));
 }
-
-// Programmatic dependent launch: a stage kernel loads its tables (constant over the
-// time loop) while the launch before it drains, then waits for that launch's results.
-__device__ __forceinline__ void dep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void dep_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Values that earlier launches of the loop wrote (state, kb, Z, P, slots).  Not the
 // read-only path: a launch may start before the one that writes them has ended.
@@ -837,23 +833,6 @@ __global__ void __launch_bounds__(line_threads<S, SV>(), line_blocks<T, S, SV, 1
 // ----------------------------------------------------------------------------
 // launches
 
-// Launch with or without programmatic dependence on the launch before.
-template <typename... P, typename... A>
-static void line_start(void (*kern)(P...), int blocks, int threads, size_t smem, cudaStream_t st, bool pdl, A &&...args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(unsigned(blocks));
-    cfg.blockDim = dim3(unsigned(threads));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = st;
-    cudaLaunchAttribute at = {};
-    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = pdl ? 1 : 0;
-    cudaLaunchKernelEx(&cfg, kern, std::forward<A>(args)...);
-}
-
 template <typename T, int S, int SV, int STAGE, int ADJ>
 static void line_launch(hrn_ctx *c, LineArgs<T> &L, int first, bool pdl)
 {
@@ -883,7 +862,7 @@ static void line_launch(hrn_ctx *c, LineArgs<T> &L, int first, bool pdl)
                 k_line_material<T><<<unsigned((int64_t(27) * L.nrd + 255) / 256), 256, 0, c->stream>>>(L);
                 ++c->launches;
             }
-            line_start(k_line_r<T, S>, int((int64_t(L.nrd) * S + 63) / 64), 64, 0, c->stream, pdl, L, static_cast<const T *>(STAGE == 1 ? L.x2 : L.kt));
+            chain_start(k_line_r<T, S>, int((int64_t(L.nrd) * S + 63) / 64), 64, 0, c->stream, pdl, L, static_cast<const T *>(STAGE == 1 ? L.x2 : L.kt));
             ++c->launches;
             pdl = true;
             nb_r = 0;
@@ -892,13 +871,13 @@ static void line_launch(hrn_ctx *c, LineArgs<T> &L, int first, bool pdl)
     if (nb_s + nb_r > 0) {
         static_assert(line_smem<T, S, SV, 0>() <= 48 * 1024, "k_line_a exceeds the default shared memory of a CTA");
         if (c->rd_box)
-            line_start(k_line_a<T, S, SV, STAGE, ADJ, 1>, nb_s + nb_r, NT, line_smem<T, S, SV, 1>(), c->stream, pdl, L, nb_s);
+            chain_start(k_line_a<T, S, SV, STAGE, ADJ, 1>, nb_s + nb_r, NT, line_smem<T, S, SV, 1>(), c->stream, pdl, L, nb_s);
         else
-            line_start(k_line_a<T, S, SV, STAGE, ADJ, 0>, nb_s + nb_r, NT, line_smem<T, S, SV, 0>(), c->stream, pdl, L, nb_s);
+            chain_start(k_line_a<T, S, SV, STAGE, ADJ, 0>, nb_s + nb_r, NT, line_smem<T, S, SV, 0>(), c->stream, pdl, L, nb_s);
         ++c->launches;
     }
     const int nb_u = (L.nun + NPB - 1) / NPB;
-    if (nb_u > 0) line_start(k_line_b<T, S, SV, STAGE, ADJ>, nb_u, NT, 0, c->stream, nb_s + nb_r > 0 || pdl, L);
+    if (nb_u > 0) chain_start(k_line_b<T, S, SV, STAGE, ADJ>, nb_u, NT, 0, c->stream, nb_s + nb_r > 0 || pdl, L);
     // the caller counts one launch per stage
 }
 
