@@ -41,7 +41,6 @@ constexpr int kM = 128;           // voxels per tile (MMA M)
 constexpr int kThreads = 128;     // one warpgroup: warp w reads TMEM lanes 32w..32w+31
 constexpr int kTmemCols = 32;     // smallest TMEM allocation; the accumulator uses 16 columns
 constexpr int kWgSteps = 8;       // K steps (16 voxels each) staged per round of the weight-gradient kernel
-constexpr int kWgChunk = 1024;    // voxels of one weight-gradient CTA
 
 struct Grid {
     int nz, ny, nx;
@@ -328,6 +327,18 @@ __global__ void __launch_bounds__(kPrepThreads) k_conv_prepare(int cin, int cout
     }
 }
 
+// Rounds of a weight-gradient CTA.  A round waits for its gathers and its MMAs in turn, so a
+// CTA's time is its rounds, and the six that fit an SM (shared memory) cover for each other:
+// up to twelve rounds the chunks are sized to one wave of 222 x 4 CTAs (41x81x81 voxels: ten
+// rounds, 88 us, where eight filled 1.2 waves, 105 us); beyond that, where the last wave is a
+// small part, eight.
+constexpr int kWgVox = kWgSteps * 16;
+int wgrad_rounds(int V)
+{
+    const int r = ((V + kWgVox - 1) / kWgVox + 221) / 222;
+    return r <= 12 ? r : 8;
+}
+
 // Weight gradient, partial sums of one chunk of voxels for one M tile of 8 taps:
 //   part[chunk][mt * 128 + (tap - 8 mt) * 16 + ci][co] = sum_v x[v + off(tap)][ci] gz[v][co]
 // Both operands are MN-major (the GEMM's K runs over voxels): core matrix
@@ -335,7 +346,7 @@ __global__ void __launch_bounds__(kPrepThreads) k_conv_prepare(int cin, int cout
 __global__ void __launch_bounds__(kThreads) k_conv_wgrad_tc(Grid g, const __nv_bfloat16 *__restrict__ x,
                                                             const float *__restrict__ gy,
                                                             const __nv_bfloat16 *__restrict__ y_act, int relu,
-                                                            float *__restrict__ part, int *__restrict__ err)
+                                                            float *__restrict__ part, int *__restrict__ err, int nround)
 {
     extern __shared__ __align__(1024) unsigned char smem[];
     unsigned char *As = smem;                         // kWgSteps x 4096
@@ -344,7 +355,7 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad_tc(Grid g, const __nv_b
     uint32_t *s_taddr = reinterpret_cast<uint32_t *>(bar + 1);
     const int V = g.size();
     const int mt = blockIdx.x, chunk = blockIdx.y;
-    const int c0 = chunk * kWgChunk;
+    const int c0 = chunk * nround * kWgVox;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) mbar_init(bar);
     if (warp == 0) tmem_alloc(s_taddr);
@@ -353,12 +364,10 @@ __global__ void __launch_bounds__(kThreads) k_conv_wgrad_tc(Grid g, const __nv_b
     fence_after();
     const uint32_t taddr = *s_taddr;
     constexpr uint32_t idesc = instr_desc(kM, kC, 1, 1);
-    constexpr int kRoundVox = kWgSteps * 16;
-    const int nround = kWgChunk / kRoundVox;
     bool ok = true;
     int issued = 0;
     for (int r = 0; r < nround && ok; ++r) {
-        const int vr = c0 + r * kRoundVox;
+        const int vr = c0 + r * kWgVox;
         if (vr >= V) break;
         // Thread m stages voxel vr + m (step s = m / 16, voxel kv = m % 16 of the step).
         // A: 16 M groups (tap, channel half) x 16 voxels per step; B: 2 N groups x 16 voxels.
@@ -610,7 +619,7 @@ extern "C" int hrn_cnn_conv3d_backward(int32_t cin, int32_t cout, int32_t nz, in
     if (cudaGetDevice(&dev) != cudaSuccess) return HRN_ECUDA;
     const Grid g{nz, ny, nx};
     const int V = g.size();
-    const int nchunk = (V + kWgChunk - 1) / kWgChunk;
+    const int nround = wgrad_rounds(V), nchunk = (V + nround * kWgVox - 1) / (nround * kWgVox);
     Scratch s;
     if (int rc = scratch(dev, size_t(nchunk) * 4 * kM * kC * sizeof(float), gx ? pad_bytes(g) : 0, s)) return rc;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
@@ -625,7 +634,7 @@ extern "C" int hrn_cnn_conv3d_backward(int32_t cin, int32_t cout, int32_t nz, in
                          nullptr, relu, gx, s.err);
     }
     k_conv_wgrad_tc<<<dim3(4, nchunk), kThreads, kWgSmem, st>>>(g, static_cast<const __nv_bfloat16 *>(x), gy, yb, relu,
-                                                                 s.part, s.err);
+                                                                 s.part, s.err, nround);
     const int nb = std::min((V + kBThreads / 4 - 1) / (kBThreads / 4), kBBlocks);
     k_conv_bias_part<<<nb, kBThreads, 0, st>>>(g, gy, yb, relu, s.bpart);
     k_conv_sum<<<kSumBlocks + 1, kSumThreads, 0, st>>>(cin, cout, nchunk, s.part, gw, nb, s.bpart, gb);
