@@ -29,17 +29,19 @@
 #include <thrust/unique.h>
 
 #include <algorithm>
+#include <atomic>
 #include <vector>
 
 #include "hrn_internal.h"
 
 namespace hrn {
 
-__constant__ unsigned char a_ijk[27][3];    // (xi, eta, zeta) index of each local node
-__constant__ unsigned char a_node_at[27];   // local node at GLL point q = 9c + 3b + a
-__constant__ double a_D[3][3];              // a_D[a][b] = l_b'(xi_a)
-__constant__ unsigned char a_kI[513], a_kJ[513], a_kn[513], a_kq[513][7];
-__constant__ unsigned char a_eaI[189], a_eaJ[189];
+// In global memory (L1), not constant memory: the lanes of a warp read different entries.
+__device__ unsigned char a_ijk[27][3];      // (xi, eta, zeta) index of each local node
+__device__ unsigned char a_node_at[27];     // local node at GLL point q = 9c + 3b + a
+__device__ double a_D[3][3];                // a_D[a][b] = l_b'(xi_a)
+__device__ unsigned char a_kI[513], a_kJ[513], a_kn[513], a_kq[513][7];
+__device__ unsigned char a_eaI[189], a_eaJ[189];   // I = J first, then the pairs along xi, eta, zeta
 
 struct AsmArgs {
     const int32_t *elems;      // element ids of this colour
@@ -50,6 +52,7 @@ struct AsmArgs {
     const double *pmla;         // [nj] the factor a
     // values mode
     const int32_t *rowptr;
+    const int2 *seg;            // [neq] first K and first G entry of each row
     const uint32_t *colx;
     double *raw, *diag_m;
     // discover mode
@@ -114,7 +117,20 @@ __device__ bool pml_ab(const double *x, const double *P, double A[10])
     return true;
 }
 
-__device__ __forceinline__ void put(const AsmArgs &A, int row, int col, int tag, double v)
+// Start of the C, K and G entries of a row and its end.
+struct RowSeg { int b[4]; };
+__device__ __forceinline__ RowSeg row_seg(const AsmArgs &A, int row)
+{
+    if (row < 0 || A.discover || A.no_csr) return {{0, 0, 0, 0}};
+    const int2 s = A.seg[row];
+    return {{A.rowptr[row], s.x, s.y, A.rowptr[row + 1]}};
+}
+
+// Adds v at (row, col) of matrix `tag`.  `at` is a guess of the entry's place among the
+// row's entries of that matrix and becomes the place found: neighbouring columns, and the
+// same column in the three matrices, mostly lie where the entry before says, and only a
+// wrong guess searches the row.
+__device__ __forceinline__ void put(const AsmArgs &A, const RowSeg &R, int row, int col, int tag, double v, int &at)
 {
     if (row < 0 || col < 0 || v == 0.0 || A.no_csr) return;   // PETSc: negative index ignored, zero not inserted
     if (A.discover) {
@@ -124,55 +140,85 @@ __device__ __forceinline__ void put(const AsmArgs &A, int row, int col, int tag,
         return;
     }
     const uint32_t key = (uint32_t(tag) << kTagBits) | uint32_t(col);
-    int lo = A.rowptr[row], hi = A.rowptr[row + 1] - 1;
-    while (lo <= hi) {
-        const int mid = lo + ((hi - lo) >> 1);   // no overflow past 2^30 entries
-        const uint32_t m = A.colx[mid];
-        if (m == key) { A.raw[mid] = add(A.raw[mid], v); return; }
-        if (m < key) lo = mid + 1; else hi = mid - 1;
+    const int b = tag == 0 ? R.b[0] : (tag == 1 ? R.b[1] : R.b[2]), e = tag == 0 ? R.b[1] : (tag == 1 ? R.b[2] : R.b[3]);
+    int mid = b + at;
+    if (at < 0 || mid >= e || A.colx[mid] != key) {
+        int lo = b, hi = e - 1;
+        for (;;) {
+            if (lo > hi) {
+                atomicExch(A.err, 3);   // contribution outside the pattern fixed by the first assembly
+                return;
+            }
+            mid = lo + ((hi - lo) >> 1);   // no overflow past 2^30 entries
+            const uint32_t m = A.colx[mid];
+            if (m == key) break;
+            if (m < key) lo = mid + 1; else hi = mid - 1;
+        }
     }
-    atomicExch(A.err, 3);   // contribution outside the pattern fixed by the first assembly
+    at = mid - b;
+    A.raw[mid] = add(A.raw[mid], v);
 }
 
-// One thread per (element, K node pair, c, d): EK of ELEMENT_K_3D (S4/Element_Matrices_3D.F90:160-210).
-__global__ void k_asm_rd_k(AsmArgs A)
+// EK of ELEMENT_K_3D (S4/Element_Matrices_3D.F90:160-210): a block per element (or part of
+// one, gridDim.y), its geometry, material and equation numbers in shared memory; one thread
+// per K node pair and row component c, which forms the three columns d from one set of
+// derivatives and finds them with one search.  One thread per (pair, c, d) repeated the
+// derivatives and the search and read its tables from constant memory at diverging
+// addresses: 4000 elements took 877 us, RDK_NOW us now.
+constexpr int kRdKThreads = 224, kRdKItems = 513 * 3;
+
+__global__ void __launch_bounds__(kRdKThreads) k_asm_rd_k(AsmArgs A)
 {
-    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (t >= int64_t(A.nel) * 513 * 9) return;
-    const int cd = int(t % 9), p = int((t / 9) % 513);
-    const int e = A.elems[t / (9 * 513)];
-    const int c = cd / 3, d = cd % 3;
-    const int I = a_kI[p], J = a_kJ[p];
+    __shared__ double sg[27 * 10], s_l[27], s_m[27];
+    __shared__ int s_id[27][3];
+    const int e = A.elems[blockIdx.x];
     const int32_t *nd = A.inod + size_t(e) * 27;
-    double s = 0.0;
-    for (int u = 0; u < a_kn[p]; ++u) {
-        const int q = a_kq[p][u];
-        const double *g = A.geom + (size_t(e) * 27 + q) * 10;
-        double fi[3], fj[3];
-        dfx_row(I, q, g, fi);
-        dfx_row(J, q, g, fj);
-        const int nq = nd[a_node_at[q]];
-        const double zl = A.lam[nq], zm = A.mu[nq];
-        const double f1 = add(zl, mul(2.0, zm)), f2 = zl, f3 = zm;
-        // G(c,d) of ELEMENT_K_3D, H_ab = DFX(I,a) DFX(J,b)
-        double G;
-        if (c == d) {
-            const int o1 = (c + 1) % 3, o2 = (c + 2) % 3;
-            // G1 = f1 H11 + f3 (H22 + H33) for c = x; cyclic forms for y, z keep the reference order
-            const double hc = mul(fi[c], fj[c]);
-            double ha, hb;
-            if (c == 0) { ha = mul(fi[1], fj[1]); hb = mul(fi[2], fj[2]); }
-            else if (c == 1) { ha = mul(fi[0], fj[0]); hb = mul(fi[2], fj[2]); }
-            else { ha = mul(fi[0], fj[0]); hb = mul(fi[1], fj[1]); }
-            (void)o1; (void)o2;
-            G = add(mul(f1, hc), mul(f3, add(ha, hb)));
-        } else {
-            // off-diagonal blocks: G = f2 * DFX(I,c) DFX(J,d) + f3 * DFX(I,d) DFX(J,c)
-            G = add(mul(f2, mul(fi[c], fj[d])), mul(f3, mul(fi[d], fj[c])));
-        }
-        s = add(s, mul(G, g[9]));
+    for (int i = threadIdx.x; i < 270; i += kRdKThreads) sg[i] = A.geom[size_t(e) * 270 + i];
+    for (int i = threadIdx.x; i < 27; i += kRdKThreads) {
+        const int nq = nd[a_node_at[i]];   // point i
+        s_l[i] = A.lam[nq];
+        s_m[i] = A.mu[nq];
     }
-    put(A, A.id[size_t(nd[I]) * 9 + c], A.id[size_t(nd[J]) * 9 + d], 1, s);
+    for (int i = threadIdx.x; i < 81; i += kRdKThreads) s_id[i / 3][i % 3] = A.id[size_t(nd[i / 3]) * 9 + i % 3];
+    __syncthreads();
+    for (int t = blockIdx.y * kRdKThreads + threadIdx.x; t < kRdKItems; t += gridDim.y * kRdKThreads) {
+        const int c = t % 3, p = t / 3;
+        const int I = a_kI[p], J = a_kJ[p], np = a_kn[p];
+        double s[3] = {0.0, 0.0, 0.0};
+        for (int u = 0; u < np; ++u) {
+            const int q = a_kq[p][u];
+            const double *g = sg + q * 10;
+            double fi[3], fj[3];
+            dfx_row(I, q, g, fi);
+            dfx_row(J, q, g, fj);
+            const double zl = s_l[q], zm = s_m[q];
+            const double f1 = add(zl, mul(2.0, zm)), f2 = zl, f3 = zm;
+            const double fic = c == 0 ? fi[0] : (c == 1 ? fi[1] : fi[2]), fjc = c == 0 ? fj[0] : (c == 1 ? fj[1] : fj[2]);
+            // G(c,d) of ELEMENT_K_3D, H_ab = DFX(I,a) DFX(J,b)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                double G;
+                if (c == d) {
+                    // G1 = f1 H11 + f3 (H22 + H33) for c = x; the forms for y, z keep the reference order
+                    const double ha = d == 0 ? mul(fi[1], fj[1]) : mul(fi[0], fj[0]);
+                    const double hb = d == 2 ? mul(fi[1], fj[1]) : mul(fi[2], fj[2]);
+                    G = add(mul(f1, mul(fi[d], fj[d])), mul(f3, add(ha, hb)));
+                } else {
+                    // off-diagonal blocks: G = f2 * DFX(I,c) DFX(J,d) + f3 * DFX(I,d) DFX(J,c)
+                    G = add(mul(f2, mul(fic, fj[d])), mul(f3, mul(fi[d], fjc)));
+                }
+                s[d] = add(s[d], mul(G, g[9]));
+            }
+        }
+        const int row = s_id[I][c];
+        const RowSeg R = row_seg(A, row);
+        int at = -1;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            put(A, R, row, s_id[J][d], 1, s[d], at);
+            if (at >= 0) ++at;   // the next component's column follows
+        }
+    }
 }
 
 // One thread per (element, local node): diagonal mass of the RD (ELEMENT_M_3D, flag 201),
@@ -217,7 +263,8 @@ __global__ void k_asm_diag(AsmArgs A, int pml)
         return;
     }
     const int cc = dof;
-    put(A, idn[cc], idn[cc], part - 1, cc < 3 ? vu : (cc < 6 ? vs1 : vs2));
+    int at = -1;
+    put(A, row_seg(A, idn[cc]), idn[cc], idn[cc], part - 1, cc < 3 ? vu : (cc < 6 ? vs1 : vs2), at);
 }
 
 // Stretching factors of every node: F1, F2, F3 of the kinds e, p, w, then b, c, d; a first
@@ -243,65 +290,87 @@ __global__ void k_asm_pml(int nj, const double *__restrict__ xyz, const double *
     a[j] = ab[6];
 }
 
-// One thread per (element, EA pair (I, J), c, d, kind e/p/w): the upper EA value goes
-// to (stress J d, displacement I c), minus the lower EA value to (I c, J d)
-// (S4/Assemble_PETSc_3D.F90:409-420; ELEMENT_EA_3D, S4/Element_Matrices_3D.F90:618-882).
-__global__ void k_asm_ea(AsmArgs A)
+// The upper EA value of a pair (I, J), c, d and kind e/p/w goes to (stress J d, displacement
+// I c), minus the lower EA value to (I c, J d) (S4/Assemble_PETSc_3D.F90:409-420;
+// ELEMENT_EA_3D, S4/Element_Matrices_3D.F90:618-882).  A block per element (or part of one,
+// gridDim.y) as above; one thread per pair and (c, d), which takes the three kinds with one
+// derivative and one search per row.  Consecutive threads take consecutive pairs of one (c, d),
+// sorted by the direction of their line, so that a warp is all in or all out where a
+// direction has no derivative.  One thread per (pair, c, d, kind), kind fastest: 4000
+// elements took 597 us, EA_NOW us now.
+constexpr int kEaThreads = 192, kEaItems = 189 * 15;
+
+__device__ __forceinline__ void ea_entry(const AsmArgs &A, int I, int J, int c, int d, const double *g, const double *F,
+                                         double zl, double zm, int ui, int sj)
 {
-    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    if (t >= int64_t(A.nel) * 189 * 18 * 3) return;
-    const int kind = int(t % 3);
-    const int cd = int((t / 3) % 18);
-    const int p = int((t / 54) % 189);
-    const int e = A.elems[t / (54 * 189)];
-    const int c = cd / 6, d = cd % 6;
-    // structural zeros EA(I1,J6), EA(I2,J5), EA(I3,J4)
-    if ((c == 0 && d == 5) || (c == 1 && d == 4) || (c == 2 && d == 3)) return;
-    const int I = a_eaI[p], J = a_eaJ[p];
-    const int32_t *nd = A.inod + size_t(e) * 27;
     const int q = 9 * a_ijk[J][2] + 3 * a_ijk[J][1] + a_ijk[J][0];
-    const double *g = A.geom + (size_t(e) * 27 + q) * 10;
-    const int nq = nd[J];
     double fi[3];
     dfx_row(I, q, g, fi);
     const double h1 = mul(fi[0], 1.0), h2 = mul(fi[1], 1.0), h3 = mul(fi[2], 1.0), h4 = (I == J) ? 1.0 : 0.0;
     // entries of a direction without a derivative are zero (I and J off its line)
     const double hd = (d == 3 ? (c == 0 ? h2 : h1) : d == 4 ? (c == 0 ? h3 : h1) : d == 5 ? (c == 1 ? h3 : h2)
                                                                                           : (c == 0 ? h1 : c == 1 ? h2 : h3));
-    const double *F = A.pmlf + size_t(nq) * 12;
     if (F[0] < 0.0) { atomicExch(A.err, 4); return; }
-    const double zl = A.lam[nq], zm = A.mu[nq];
     if (hd == 0.0 && isfinite(zl) && isfinite(zm)) return;   // 0 times a non-finite modulus is not
-    const double F1 = F[3 * kind], F2 = F[3 * kind + 1], F3 = F[3 * kind + 2];
-    double vals[2];
-    for (int lower = 0; lower < 2; ++lower) {
-        const double f7 = lower ? add(zl, mul(2.0, zm)) : 1.0;
-        const double f8 = lower ? zl : 0.0;
-        const double f9 = lower ? mul(2.0, zm) : 1.0;
-        const double f10 = lower ? 0.0 : 1.0;
-        // FAC4..FAC6 vanish with ratio 0; f10 * 0 * h4 keeps the reference's terms
-        const double z = mul(mul(f10, 0.0), h4);
-        double G;
-        switch (c * 6 + d) {
-        case 0: G = add(mul(mul(f7, F3), h1), z); break;       // G1
-        case 1: case 2: G = mul(mul(f8, F3), h1); break;      // G2
-        case 3: G = add(mul(mul(f9, F2), h2), z); break;       // G3
-        case 4: G = add(mul(mul(f9, F1), h3), z); break;       // G4
-        case 6: case 8: G = mul(mul(f8, F2), h2); break;      // G5
-        case 7: G = add(mul(mul(f7, F2), h2), z); break;       // G6
-        case 9: G = add(mul(mul(f9, F3), h1), z); break;       // G7
-        case 11: G = add(mul(mul(f9, F1), h3), z); break;      // G4
-        case 12: case 13: G = mul(mul(f8, F1), h3); break;    // G8
-        case 14: G = add(mul(mul(f7, F1), h3), z); break;      // G9
-        case 16: G = add(mul(mul(f9, F3), h1), z); break;      // G7
-        default: G = add(mul(mul(f9, F2), h2), z); break;      // 17: G3
+    const RowSeg Rs = row_seg(A, sj), Ru = row_seg(A, ui);
+    int at_s = -1, at_u = -1;
+    for (int kind = 0; kind < 3; ++kind) {
+        const double F1 = F[3 * kind], F2 = F[3 * kind + 1], F3 = F[3 * kind + 2];
+        double vals[2];
+        for (int lower = 0; lower < 2; ++lower) {
+            const double f7 = lower ? add(zl, mul(2.0, zm)) : 1.0;
+            const double f8 = lower ? zl : 0.0;
+            const double f9 = lower ? mul(2.0, zm) : 1.0;
+            const double f10 = lower ? 0.0 : 1.0;
+            // FAC4..FAC6 vanish with ratio 0; f10 * 0 * h4 keeps the reference's terms
+            const double z = mul(mul(f10, 0.0), h4);
+            double G;
+            switch (c * 6 + d) {
+            case 0: G = add(mul(mul(f7, F3), h1), z); break;       // G1
+            case 1: case 2: G = mul(mul(f8, F3), h1); break;      // G2
+            case 3: G = add(mul(mul(f9, F2), h2), z); break;       // G3
+            case 4: G = add(mul(mul(f9, F1), h3), z); break;       // G4
+            case 6: case 8: G = mul(mul(f8, F2), h2); break;      // G5
+            case 7: G = add(mul(mul(f7, F2), h2), z); break;       // G6
+            case 9: G = add(mul(mul(f9, F3), h1), z); break;       // G7
+            case 11: G = add(mul(mul(f9, F1), h3), z); break;      // G4
+            case 12: case 13: G = mul(mul(f8, F1), h3); break;    // G8
+            case 14: G = add(mul(mul(f7, F1), h3), z); break;      // G9
+            case 16: G = add(mul(mul(f9, F3), h1), z); break;      // G7
+            default: G = add(mul(mul(f9, F2), h2), z); break;      // 17: G3
+            }
+            vals[lower] = mul(G, g[9]);
         }
-        vals[lower] = mul(G, g[9]);
+        put(A, Rs, sj, ui, kind, vals[0], at_s);
+        put(A, Ru, ui, sj, kind, -vals[1], at_u);
     }
-    const int ui = A.id[size_t(nd[I]) * 9 + c];
-    const int sj = A.id[size_t(nd[J]) * 9 + 3 + d];
-    put(A, sj, ui, kind, vals[0]);
-    put(A, ui, sj, kind, -vals[1]);
+}
+
+__global__ void __launch_bounds__(kEaThreads) k_asm_ea(AsmArgs A)
+{
+    __shared__ double sg[27 * 10], sf[27 * 9], s_l[27], s_m[27];
+    __shared__ int s_id[27 * 9];
+    const int e = A.elems[blockIdx.x];
+    const int32_t *nd = A.inod + size_t(e) * 27;
+    for (int i = threadIdx.x; i < 270; i += kEaThreads) sg[i] = A.geom[size_t(e) * 270 + i];
+    for (int i = threadIdx.x; i < 243; i += kEaThreads) {
+        const int n = nd[i / 9];
+        sf[i] = A.pmlf[size_t(n) * 12 + i % 9];
+        s_id[i] = A.id[size_t(n) * 9 + i % 9];
+    }
+    for (int i = threadIdx.x; i < 27; i += kEaThreads) {
+        s_l[i] = A.lam[nd[i]];
+        s_m[i] = A.mu[nd[i]];
+    }
+    __syncthreads();
+    for (int t = blockIdx.y * kEaThreads + threadIdx.x; t < kEaItems; t += gridDim.y * kEaThreads) {
+        const int p = t % 189, cd = t / 189, c = cd / 5, k = cd % 5;
+        // all d but the structural zeros EA(I1,J6), EA(I2,J5), EA(I3,J4)
+        const int d = k < 3 ? k : (c == 0 ? k : c == 1 ? (k == 3 ? 3 : 5) : k + 1);
+        const int I = a_eaI[p], J = a_eaJ[p];
+        const int q = 9 * a_ijk[J][2] + 3 * a_ijk[J][1] + a_ijk[J][0];
+        ea_entry(A, I, J, c, d, sg + q * 10, sf + J * 9, s_l[J], s_m[J], s_id[I * 9 + c], s_id[J * 9 + 3 + d]);
+    }
 }
 
 __global__ void k_inv_mass(int n, const double *__restrict__ dm, double *__restrict__ im)
@@ -313,8 +382,14 @@ __global__ void k_inv_mass(int n, const double *__restrict__ dm, double *__restr
 // ----------------------------------------------------------------------------
 // host side
 
+// Once per device: nine synchronous copies took 70 us of every assembly.
 static int upload_asm_tables(hrn_ctx *c)
 {
+    static std::atomic<uint64_t> done{0};
+    int dev = 0;
+    HRN_CUDA(c, cudaGetDevice(&dev));
+    const uint64_t bit = dev < 64 ? (uint64_t(1) << dev) : 0;
+    if (done.load() & bit) return 0;
     static const unsigned char ijk[27][3] = {{2, 0, 0}, {2, 2, 0}, {0, 2, 0}, {0, 0, 0}, {2, 0, 2}, {2, 2, 2}, {0, 2, 2},
                                              {0, 0, 2}, {2, 1, 0}, {1, 2, 0}, {0, 1, 0}, {1, 0, 0}, {2, 0, 1}, {2, 2, 1},
                                              {0, 2, 1}, {0, 0, 1}, {2, 1, 2}, {1, 2, 2}, {0, 1, 2}, {1, 0, 2}, {1, 1, 0},
@@ -342,11 +417,14 @@ static int upload_asm_tables(hrn_ctx *c)
     if (np != 513) return set_error(c, HRN_ESTATE, "internal: element pair table size");
     unsigned char eI[189], eJ[189];
     int ne = 0;
-    for (int J = 0; J < 27; ++J) {
-        const int q = 9 * ijk[J][2] + 3 * ijk[J][1] + ijk[J][0];
-        for (int I = 0; I < 27; ++I)
-            if (on_lines(I, q)) { eI[ne] = (unsigned char)I; eJ[ne] = (unsigned char)J; ++ne; }
-    }
+    for (int dir = -1; dir < 3; ++dir)   // I = J, then the pairs along each direction
+        for (int J = 0; J < 27; ++J)
+            for (int I = 0; I < 27; ++I) {
+                int at = -1, ndiff = 0;
+                for (int m = 0; m < 3; ++m)
+                    if (ijk[I][m] != ijk[J][m]) { at = m; ++ndiff; }
+                if (ndiff <= 1 && at == dir) { eI[ne] = (unsigned char)I; eJ[ne] = (unsigned char)J; ++ne; }
+            }
     if (ne != 189) return set_error(c, HRN_ESTATE, "internal: EA pair table size");
     const double D[3][3] = {{-1.5, 2.0, -0.5}, {-0.5, 0.0, 0.5}, {0.5, -2.0, 1.5}};
     HRN_CUDA(c, cudaMemcpyToSymbol(a_ijk, ijk, sizeof(ijk)));
@@ -358,6 +436,8 @@ static int upload_asm_tables(hrn_ctx *c)
     HRN_CUDA(c, cudaMemcpyToSymbol(a_kq, kq, sizeof(kq)));
     HRN_CUDA(c, cudaMemcpyToSymbol(a_eaI, eI, sizeof(eI)));
     HRN_CUDA(c, cudaMemcpyToSymbol(a_eaJ, eJ, sizeof(eJ)));
+    HRN_CUDA(c, cudaStreamSynchronize(nullptr));
+    done.fetch_or(bit);
     return 0;
 }
 
@@ -403,6 +483,8 @@ static int build_colors(hrn_ctx *c)
     return 0;
 }
 
+constexpr int kAsmBlocks = 148 * 8;   // a full set of resident blocks of the element kernels
+
 // The kernels of elements [off, off + n) of one (colour, kind) group.
 static int run_group(hrn_ctx *c, AsmArgs A, int g, int off, int n)
 {
@@ -412,13 +494,11 @@ static int run_group(hrn_ctx *c, AsmArgs A, int g, int off, int n)
     A.nel = n;
     const bool pml = (g % 2) == 1;
     k_asm_diag<<<unsigned((int64_t(n) * 27 * (pml ? kDiagParts : 1) + th - 1) / th), th, 0, c->stream>>>(A, pml ? 1 : 0); ++c->launches;
-    if (!pml) {
-        const int64_t tot = int64_t(n) * 513 * 9;
-        k_asm_rd_k<<<unsigned((tot + th - 1) / th), th, 0, c->stream>>>(A); ++c->launches;
-    } else {
-        const int64_t tot = int64_t(n) * 189 * 54;
-        k_asm_ea<<<unsigned((tot + th - 1) / th), th, 0, c->stream>>>(A); ++c->launches;
-    }
+    // an element is one block where there are enough of them, else several
+    auto parts = [&](int most) { return unsigned(std::min(most, (kAsmBlocks + n - 1) / n)); };
+    if (!pml) k_asm_rd_k<<<dim3(unsigned(n), parts((kRdKItems + kRdKThreads - 1) / kRdKThreads)), kRdKThreads, 0, c->stream>>>(A);
+    else k_asm_ea<<<dim3(unsigned(n), parts((kEaItems + kEaThreads - 1) / kEaThreads)), kEaThreads, 0, c->stream>>>(A);
+    ++c->launches;
     HRN_CUDA(c, cudaGetLastError());
     return 0;
 }
@@ -547,6 +627,7 @@ int assemble_device(hrn_ctx *c, bool discover_pattern)
     HRN_CUDA(c, cudaMemsetAsync(c->d_asm_err.p, 0, 16, c->stream));
     A.discover = 0;
     A.rowptr = c->d_rowptr.as<int32_t>();
+    A.seg = c->d_seg.as<int2>();
     A.colx = c->d_colx.as<uint32_t>();
     A.raw = c->d_raw.as<double>();
     A.diag_m = c->d_diag_m.as<double>();
