@@ -57,7 +57,6 @@ struct AsmArgs {
     double *raw, *diag_m;
     // discover mode
     int discover;
-    int no_csr;                 // matrix-free operator: DIAG_M only, no CSR entries
     unsigned long long *count;
     unsigned long long cap;
     uint64_t *keys;
@@ -121,7 +120,7 @@ __device__ bool pml_ab(const double *x, const double *P, double A[10])
 struct RowSeg { int b[4]; };
 __device__ __forceinline__ RowSeg row_seg(const AsmArgs &A, int row)
 {
-    if (row < 0 || A.discover || A.no_csr) return {{0, 0, 0, 0}};
+    if (row < 0 || A.discover) return {{0, 0, 0, 0}};
     const int2 s = A.seg[row];
     return {{A.rowptr[row], s.x, s.y, A.rowptr[row + 1]}};
 }
@@ -132,7 +131,7 @@ __device__ __forceinline__ RowSeg row_seg(const AsmArgs &A, int row)
 // wrong guess searches the row.
 __device__ __forceinline__ void put(const AsmArgs &A, const RowSeg &R, int row, int col, int tag, double v, int &at)
 {
-    if (row < 0 || col < 0 || v == 0.0 || A.no_csr) return;   // PETSc: negative index ignored, zero not inserted
+    if (row < 0 || col < 0 || v == 0.0) return;   // PETSc: negative index ignored, zero not inserted
     if (A.discover) {
         const unsigned long long k = atomicAdd(A.count, 1ull);
         if (k < A.cap) A.keys[k] = (uint64_t(uint32_t(row)) << 32) | (uint64_t(tag) << kTagBits) | uint64_t(col);
@@ -159,39 +158,70 @@ __device__ __forceinline__ void put(const AsmArgs &A, const RowSeg &R, int row, 
     A.raw[mid] = add(A.raw[mid], v);
 }
 
-// EK of ELEMENT_K_3D (S4/Element_Matrices_3D.F90:160-210): a block per element (or part of
-// one, gridDim.y), its geometry, material and equation numbers in shared memory; one thread
+// Shared memory of an element's block.
+struct AsmElem {
+    double g[27 * 10], l[27], m[27], f[27 * 9];   // geometry, material, stretching factors
+    int id[27 * 9];
+};
+constexpr int kAsmThreads = 224;
+
+// Diagonal mass of a regular-domain node (ELEMENT_M_3D, flag 201): (RO * FN(I) FN(I)) * FAC0.
+__device__ __forceinline__ void mass_rd(const AsmArgs &A, const int32_t *idn, double rho, double fac0)
+{
+    if (A.discover) return;
+    const double v = mul(mul(rho, 1.0), fac0);
+    for (int cc = 0; cc < 3; ++cc)
+        if (idn[cc] >= 0) A.diag_m[idn[cc]] = add(A.diag_m[idn[cc]], v);
+}
+
+// EM_a (u) and EN_a (s) of a PML node (flags 202, 301), f the factor a.
+__device__ __forceinline__ void mass_pml(const AsmArgs &A, const int32_t *idn, double rho, double f, double fac0)
+{
+    if (A.discover) return;
+    const double vu = mul(mul(mul(rho, f), 1.0), fac0);
+    const double vs1 = mul(mul(f, 1.0), fac0);
+    const double vs2 = mul(mul(mul(2.0, f), 1.0), fac0);
+    for (int cc = 0; cc < 3; ++cc)
+        if (idn[cc] >= 0) A.diag_m[idn[cc]] = add(A.diag_m[idn[cc]], vu);
+    for (int cc = 0; cc < 6; ++cc)
+        if (idn[3 + cc] >= 0) A.diag_m[idn[3 + cc]] = add(A.diag_m[idn[3 + cc]], cc < 3 ? vs1 : vs2);
+}
+
+// EK of ELEMENT_K_3D (S4/Element_Matrices_3D.F90:160-210) and the mass: a block per element
+// (or part of one), its geometry, material and equation numbers in shared memory; one thread
 // per K node pair and row component c, which forms the three columns d from one set of
 // derivatives and finds them with one search.  One thread per (pair, c, d) repeated the
 // derivatives and the search and read its tables from constant memory at diverging
-// addresses: 4000 elements took 877 us, RDK_NOW us now.
-constexpr int kRdKThreads = 224, kRdKItems = 513 * 3;
+// addresses: 4000 elements took 877 us, 475 us in this form.
+constexpr int kRdItems = 513 * 3 + 27;
 
-__global__ void __launch_bounds__(kRdKThreads) k_asm_rd_k(AsmArgs A)
+__device__ __forceinline__ void element_rd(const AsmArgs &A, AsmElem &S, int e, int part, int parts)
 {
-    __shared__ double sg[27 * 10], s_l[27], s_m[27];
-    __shared__ int s_id[27][3];
-    const int e = A.elems[blockIdx.x];
     const int32_t *nd = A.inod + size_t(e) * 27;
-    for (int i = threadIdx.x; i < 270; i += kRdKThreads) sg[i] = A.geom[size_t(e) * 270 + i];
-    for (int i = threadIdx.x; i < 27; i += kRdKThreads) {
+    for (int i = threadIdx.x; i < 270; i += kAsmThreads) S.g[i] = A.geom[size_t(e) * 270 + i];
+    for (int i = threadIdx.x; i < 27; i += kAsmThreads) {
         const int nq = nd[a_node_at[i]];   // point i
-        s_l[i] = A.lam[nq];
-        s_m[i] = A.mu[nq];
+        S.l[i] = A.lam[nq];
+        S.m[i] = A.mu[nq];
     }
-    for (int i = threadIdx.x; i < 81; i += kRdKThreads) s_id[i / 3][i % 3] = A.id[size_t(nd[i / 3]) * 9 + i % 3];
+    for (int i = threadIdx.x; i < 81; i += kAsmThreads) S.id[i] = A.id[size_t(nd[i / 3]) * 9 + i % 3];
     __syncthreads();
-    for (int t = blockIdx.y * kRdKThreads + threadIdx.x; t < kRdKItems; t += gridDim.y * kRdKThreads) {
+    for (int t = part * kAsmThreads + threadIdx.x; t < kRdItems; t += parts * kAsmThreads) {
+        if (t >= 513 * 3) {
+            const int I = t - 513 * 3, q = 9 * a_ijk[I][2] + 3 * a_ijk[I][1] + a_ijk[I][0];
+            mass_rd(A, S.id + 3 * I, A.rho[e], S.g[q * 10 + 9]);
+            continue;
+        }
         const int c = t % 3, p = t / 3;
         const int I = a_kI[p], J = a_kJ[p], np = a_kn[p];
         double s[3] = {0.0, 0.0, 0.0};
         for (int u = 0; u < np; ++u) {
             const int q = a_kq[p][u];
-            const double *g = sg + q * 10;
+            const double *g = S.g + q * 10;
             double fi[3], fj[3];
             dfx_row(I, q, g, fi);
             dfx_row(J, q, g, fj);
-            const double zl = s_l[q], zm = s_m[q];
+            const double zl = S.l[q], zm = S.m[q];
             const double f1 = add(zl, mul(2.0, zm)), f2 = zl, f3 = zm;
             const double fic = c == 0 ? fi[0] : (c == 1 ? fi[1] : fi[2]), fjc = c == 0 ? fj[0] : (c == 1 ? fj[1] : fj[2]);
             // G(c,d) of ELEMENT_K_3D, H_ab = DFX(I,a) DFX(J,b)
@@ -210,61 +240,33 @@ __global__ void __launch_bounds__(kRdKThreads) k_asm_rd_k(AsmArgs A)
                 s[d] = add(s[d], mul(G, g[9]));
             }
         }
-        const int row = s_id[I][c];
+        const int row = S.id[3 * I + c];
         const RowSeg R = row_seg(A, row);
         int at = -1;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            put(A, R, row, s_id[J][d], 1, s[d], at);
+            put(A, R, row, S.id[3 * J + d], 1, s[d], at);
             if (at >= 0) ++at;   // the next component's column follows
         }
     }
 }
 
-// One thread per (element, local node): diagonal mass of the RD (ELEMENT_M_3D, flag 201),
-// and for PML elements the diagonal blocks EM_a..d (flags 202-205), EN_a..d (301-304).
-// One thread a factor and DOF for the PML's (kDiagParts: the mass, then 9 DOF of b, c, d),
-// each with its own search in the pattern: 27 searches in sequence took 80 us a colour.
-constexpr int kDiagParts = 1 + 3 * 9;
-__global__ void k_asm_diag(AsmArgs A, int pml)
+// DIAG_M alone, one thread per (element, local node).
+__global__ void k_asm_mass(AsmArgs A, int pml)
 {
-    const int64_t tt = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-    const int parts = pml ? (A.no_csr ? 1 : kDiagParts) : 1;
-    const int64_t t = tt / parts;
+    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
     if (t >= int64_t(A.nel) * 27) return;
-    const int I = int(t % 27);
-    const int e = A.elems[t / 27];
-    const int k = int(tt % parts), part = k == 0 ? 0 : 1 + (k - 1) / 9, dof = k == 0 ? 0 : (k - 1) % 9;
+    const int I = int(t % 27), e = A.elems[t / 27];
     const int node = A.inod[size_t(e) * 27 + I];
     const int q = 9 * a_ijk[I][2] + 3 * a_ijk[I][1] + a_ijk[I][0];
     const double fac0 = A.geom[(size_t(e) * 27 + q) * 10 + 9];
-    const double rho = A.rho[e];
     const int32_t *idn = A.id + size_t(node) * 9;
     if (!pml) {
-        const double v = mul(mul(rho, 1.0), fac0);   // (RO * FN(I) FN(I)) * FAC0
-        if (A.discover) return;
-        for (int cc = 0; cc < 3; ++cc)
-            if (idn[cc] >= 0) A.diag_m[idn[cc]] = add(A.diag_m[idn[cc]], v);
+        mass_rd(A, idn, A.rho[e], fac0);
         return;
     }
-    const double *F = A.pmlf + size_t(node) * 12;
-    if (F[0] < 0.0) { atomicExch(A.err, 4); return; }
-    // EM_f (u) and EN_f (s) diagonal values for f = a, b, c, d
-    const double f = part == 0 ? A.pmla[node] : F[8 + part];
-    const double vu = mul(mul(mul(rho, f), 1.0), fac0);
-    const double vs1 = mul(mul(f, 1.0), fac0);
-    const double vs2 = mul(mul(mul(2.0, f), 1.0), fac0);
-    if (part == 0) {
-        if (A.discover) return;
-        for (int cc = 0; cc < 3; ++cc)
-            if (idn[cc] >= 0) A.diag_m[idn[cc]] = add(A.diag_m[idn[cc]], vu);
-        for (int cc = 0; cc < 6; ++cc)
-            if (idn[3 + cc] >= 0) A.diag_m[idn[3 + cc]] = add(A.diag_m[idn[3 + cc]], cc < 3 ? vs1 : vs2);
-        return;
-    }
-    const int cc = dof;
-    int at = -1;
-    put(A, row_seg(A, idn[cc]), idn[cc], idn[cc], part - 1, cc < 3 ? vu : (cc < 6 ? vs1 : vs2), at);
+    if (A.pmlf[size_t(node) * 12] < 0.0) { atomicExch(A.err, 4); return; }
+    mass_pml(A, idn, A.rho[e], A.pmla[node], fac0);
 }
 
 // Stretching factors of every node: F1, F2, F3 of the kinds e, p, w, then b, c, d; a first
@@ -292,13 +294,14 @@ __global__ void k_asm_pml(int nj, const double *__restrict__ xyz, const double *
 
 // The upper EA value of a pair (I, J), c, d and kind e/p/w goes to (stress J d, displacement
 // I c), minus the lower EA value to (I c, J d) (S4/Assemble_PETSc_3D.F90:409-420;
-// ELEMENT_EA_3D, S4/Element_Matrices_3D.F90:618-882).  A block per element (or part of one,
-// gridDim.y) as above; one thread per pair and (c, d), which takes the three kinds with one
+// ELEMENT_EA_3D, S4/Element_Matrices_3D.F90:618-882).  A block per element (or part of one)
+// as above; one thread per pair and (c, d), which takes the three kinds with one
 // derivative and one search per row.  Consecutive threads take consecutive pairs of one (c, d),
 // sorted by the direction of their line, so that a warp is all in or all out where a
 // direction has no derivative.  One thread per (pair, c, d, kind), kind fastest: 4000
-// elements took 597 us, EA_NOW us now.
-constexpr int kEaThreads = 192, kEaItems = 189 * 15;
+// elements took 597 us, 210 us in this form.  Behind the pairs come the diagonal blocks
+// EM_b..d, EN_b..d (flags 203-205, 302-304), one thread per node, factor and DOF, and the mass.
+constexpr int kEaPairs = 189 * 15, kEaItems = kEaPairs + 27 * 27 + 27;
 
 __device__ __forceinline__ void ea_entry(const AsmArgs &A, int I, int J, int c, int d, const double *g, const double *F,
                                          double zl, double zm, int ui, int sj)
@@ -346,31 +349,58 @@ __device__ __forceinline__ void ea_entry(const AsmArgs &A, int I, int J, int c, 
     }
 }
 
-__global__ void __launch_bounds__(kEaThreads) k_asm_ea(AsmArgs A)
+__device__ __forceinline__ void element_pml(const AsmArgs &A, AsmElem &S, int e, int part, int parts)
 {
-    __shared__ double sg[27 * 10], sf[27 * 9], s_l[27], s_m[27];
-    __shared__ int s_id[27 * 9];
-    const int e = A.elems[blockIdx.x];
     const int32_t *nd = A.inod + size_t(e) * 27;
-    for (int i = threadIdx.x; i < 270; i += kEaThreads) sg[i] = A.geom[size_t(e) * 270 + i];
-    for (int i = threadIdx.x; i < 243; i += kEaThreads) {
+    for (int i = threadIdx.x; i < 270; i += kAsmThreads) S.g[i] = A.geom[size_t(e) * 270 + i];
+    for (int i = threadIdx.x; i < 243; i += kAsmThreads) {
         const int n = nd[i / 9];
-        sf[i] = A.pmlf[size_t(n) * 12 + i % 9];
-        s_id[i] = A.id[size_t(n) * 9 + i % 9];
+        S.f[i] = A.pmlf[size_t(n) * 12 + i % 9];
+        S.id[i] = A.id[size_t(n) * 9 + i % 9];
     }
-    for (int i = threadIdx.x; i < 27; i += kEaThreads) {
-        s_l[i] = A.lam[nd[i]];
-        s_m[i] = A.mu[nd[i]];
+    for (int i = threadIdx.x; i < 27; i += kAsmThreads) {
+        S.l[i] = A.lam[nd[i]];
+        S.m[i] = A.mu[nd[i]];
     }
     __syncthreads();
-    for (int t = blockIdx.y * kEaThreads + threadIdx.x; t < kEaItems; t += gridDim.y * kEaThreads) {
-        const int p = t % 189, cd = t / 189, c = cd / 5, k = cd % 5;
-        // all d but the structural zeros EA(I1,J6), EA(I2,J5), EA(I3,J4)
-        const int d = k < 3 ? k : (c == 0 ? k : c == 1 ? (k == 3 ? 3 : 5) : k + 1);
-        const int I = a_eaI[p], J = a_eaJ[p];
-        const int q = 9 * a_ijk[J][2] + 3 * a_ijk[J][1] + a_ijk[J][0];
-        ea_entry(A, I, J, c, d, sg + q * 10, sf + J * 9, s_l[J], s_m[J], s_id[I * 9 + c], s_id[J * 9 + 3 + d]);
+    for (int t = part * kAsmThreads + threadIdx.x; t < kEaItems; t += parts * kAsmThreads) {
+        if (t < kEaPairs) {
+            const int p = t % 189, cd = t / 189, c = cd / 5, k = cd % 5;
+            // all d but the structural zeros EA(I1,J6), EA(I2,J5), EA(I3,J4)
+            const int d = k < 3 ? k : (c == 0 ? k : c == 1 ? (k == 3 ? 3 : 5) : k + 1);
+            const int I = a_eaI[p], J = a_eaJ[p];
+            const int q = 9 * a_ijk[J][2] + 3 * a_ijk[J][1] + a_ijk[J][0];
+            ea_entry(A, I, J, c, d, S.g + q * 10, S.f + J * 9, S.l[J], S.m[J], S.id[I * 9 + c], S.id[J * 9 + 3 + d]);
+            continue;
+        }
+        const int k = t - kEaPairs;
+        const bool mass = k >= 27 * 27;
+        const int I = mass ? k - 27 * 27 : k / 27, f = (k % 27) / 9, dof = k % 9;
+        const int q = 9 * a_ijk[I][2] + 3 * a_ijk[I][1] + a_ijk[I][0];
+        if (S.f[I * 9] < 0.0) { atomicExch(A.err, 4); continue; }
+        const double rho = A.rho[e], fac0 = S.g[q * 10 + 9];
+        if (mass) {
+            mass_pml(A, S.id + I * 9, rho, A.pmla[nd[I]], fac0);
+            continue;
+        }
+        const double F = A.pmlf[size_t(nd[I]) * 12 + 9 + f];   // b, c, d
+        const double v = dof < 3 ? mul(mul(mul(rho, F), 1.0), fac0) : (dof < 6 ? mul(mul(F, 1.0), fac0) : mul(mul(mul(2.0, F), 1.0), fac0));
+        const int row = S.id[I * 9 + dof];
+        int at = -1;
+        put(A, row_seg(A, row), row, row, f, v, at);
     }
+}
+
+// One colour: nrd regular-domain elements, then the PML elements, in one launch.  Elements of
+// a colour share no node and the parts of an element write different entries, so nothing
+// here depends on anything else; four launches in sequence left the chip idle between
+// them (assembly of 4x4x2: 416 us, 202 us in one; 40x40x20: 7.3 and 6.8 ms).
+__global__ void __launch_bounds__(kAsmThreads) k_asm_elements(AsmArgs A, int nrd, int parts_rd, int parts_pml)
+{
+    __shared__ AsmElem S;
+    const int b = blockIdx.x, brd = nrd * parts_rd;
+    if (b < brd) element_rd(A, S, A.elems[b / parts_rd], b % parts_rd, parts_rd);
+    else element_pml(A, S, A.elems[nrd + (b - brd) / parts_pml], (b - brd) % parts_pml, parts_pml);
 }
 
 __global__ void k_inv_mass(int n, const double *__restrict__ dm, double *__restrict__ im)
@@ -483,21 +513,19 @@ static int build_colors(hrn_ctx *c)
     return 0;
 }
 
-constexpr int kAsmBlocks = 148 * 8;   // a full set of resident blocks of the element kernels
+constexpr int kAsmBlocks = 148 * 8;   // a full set of resident blocks of the element kernel
 
-// The kernels of elements [off, off + n) of one (colour, kind) group.
-static int run_group(hrn_ctx *c, AsmArgs A, int g, int off, int n)
+// nrd regular-domain and npml PML elements from place `off` of the colour list.
+static int run_elements(hrn_ctx *c, AsmArgs A, int off, int nrd, int npml)
 {
-    const int th = 256;
+    const int n = nrd + npml;
     if (n <= 0) return 0;
-    A.elems = c->d_el_color_list.as<int32_t>() + c->color_off[g] + off;
+    A.elems = c->d_el_color_list.as<int32_t>() + off;
     A.nel = n;
-    const bool pml = (g % 2) == 1;
-    k_asm_diag<<<unsigned((int64_t(n) * 27 * (pml ? kDiagParts : 1) + th - 1) / th), th, 0, c->stream>>>(A, pml ? 1 : 0); ++c->launches;
     // an element is one block where there are enough of them, else several
-    auto parts = [&](int most) { return unsigned(std::min(most, (kAsmBlocks + n - 1) / n)); };
-    if (!pml) k_asm_rd_k<<<dim3(unsigned(n), parts((kRdKItems + kRdKThreads - 1) / kRdKThreads)), kRdKThreads, 0, c->stream>>>(A);
-    else k_asm_ea<<<dim3(unsigned(n), parts((kEaItems + kEaThreads - 1) / kEaThreads)), kEaThreads, 0, c->stream>>>(A);
+    auto parts = [&](int items) { return std::min((items + kAsmThreads - 1) / kAsmThreads, (kAsmBlocks + n - 1) / n); };
+    const int pr = parts(kRdItems), pp = parts(kEaItems);
+    k_asm_elements<<<unsigned(nrd * pr + npml * pp), kAsmThreads, 0, c->stream>>>(A, nrd, pr, pp);
     ++c->launches;
     HRN_CUDA(c, cudaGetLastError());
     return 0;
@@ -505,9 +533,9 @@ static int run_group(hrn_ctx *c, AsmArgs A, int g, int off, int n)
 
 static int run_kernels(hrn_ctx *c, AsmArgs A)
 {
-    const int ngroups = int(c->color_off.size()) - 1;   // (colour, kind) groups
-    for (int g = 0; g < ngroups; ++g)
-        if (int rc = run_group(c, A, g, 0, c->color_off[g + 1] - c->color_off[g])) return rc;
+    const std::vector<int> &off = c->color_off;   // (colour, kind) groups, regular domain first
+    for (size_t g = 0; g + 2 < off.size(); g += 2)
+        if (int rc = run_elements(c, A, off[g], off[g + 1] - off[g], off[g + 2] - off[g + 1])) return rc;
     return 0;
 }
 
@@ -524,7 +552,6 @@ static int assemble_mass_only(hrn_ctx *c, AsmArgs A)
     HRN_CUDA(c, c->d_im.alloc(size_t(c->neq) * 8));
     HRN_CUDA(c, cudaMemsetAsync(c->d_diag_m.p, 0, size_t(c->neq) * 8, c->stream));
     A.discover = 0;
-    A.no_csr = 1;
     A.diag_m = c->d_diag_m.as<double>();
     const int ngroups = int(c->color_off.size()) - 1;
     for (int g = 0; g < ngroups; ++g) {
@@ -532,7 +559,7 @@ static int assemble_mass_only(hrn_ctx *c, AsmArgs A)
         if (n == 0) continue;
         A.elems = c->d_el_color_list.as<int32_t>() + c->color_off[g];
         A.nel = n;
-        k_asm_diag<<<(n * 27 + th - 1) / th, th, 0, c->stream>>>(A, (g % 2) == 1 ? 1 : 0); ++c->launches;
+        k_asm_mass<<<(n * 27 + th - 1) / th, th, 0, c->stream>>>(A, (g % 2) == 1 ? 1 : 0); ++c->launches;
         HRN_CUDA(c, cudaGetLastError());
     }
     k_inv_mass<<<(c->neq + 255) / 256, 256, 0, c->stream>>>(c->neq, c->d_diag_m.as<double>(), c->d_im.as<double>()); ++c->launches;
@@ -591,7 +618,7 @@ int assemble_device(hrn_ctx *c, bool discover_pattern)
                 const int n = std::min(slice, ng - off);
                 A.cap = (unsigned long long)n * per;
                 HRN_CUDA(c, cudaMemsetAsync(count.p, 0, 8, c->stream));
-                if (int rc = run_group(c, A, g, off, n)) return rc;
+                if (int rc = run_elements(c, A, c->color_off[g] + off, g % 2 ? 0 : n, g % 2 ? n : 0)) return rc;
                 unsigned long long nk = 0;
                 int err = 0;
                 HRN_CUDA(c, cudaMemcpyAsync(&nk, count.p, 8, cudaMemcpyDeviceToHost, c->stream));
