@@ -953,9 +953,13 @@ static int autotune_lanes(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, const TileArgs
     if (line) {
         // Where the line operator serves the mesh it is 1.4 to 2.2 times as fast as the best
         // other variant from about 70 thousand equations up; only on the smallest meshes, where
-        // its two launches count, is the row-parallel kernel ahead (8 against 10 us a stage at
-        // 8 thousand equations).  The tables of the others need not be built.
-        if (c->have_pattern) cand = {41, 81};
+        // its two launches count, are the row-parallel kernels ahead (6 against 10 us a stage at
+        // 8 thousand equations), and which of them depends on the lanes.  The tables of the
+        // others need not be built.
+        if (c->have_pattern) {
+            if (c->neq < 100000) cand = {40, 80, 160, 41, 81, 161};
+            else cand = {41, 81};
+        }
         cand.push_back(96);
         if (c->nshot % 2 == 0) cand.push_back(97);
         if (c->nshot % 4 == 0 && c->precision == HRN_FP32) cand.push_back(98);
