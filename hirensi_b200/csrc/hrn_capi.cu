@@ -475,6 +475,7 @@ int hrn_set_mesh(hrn_ctx *c, int32_t nj, int32_t nel, int32_t neq, const double 
     c->have_elem = false;
     c->have_line = false;
     c->have_asm_pml = false;
+    c->color_off.clear();   // the colour list names the old mesh's elements
     c->line_epoch = 0;
     if (is_line_variant(c->lanes_f)) c->lanes_f = 0;   // the new mesh may not suit the line operator: tune again
     if (is_line_variant(c->lanes_a)) c->lanes_a = 0;
