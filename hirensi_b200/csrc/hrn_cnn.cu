@@ -514,10 +514,11 @@ int check(int cin, int cout, int nz, int ny, int nx)
 }
 
 // Per-device scratch of the layers (the error flag, the packed B operand, the padded
-// copy of the A source and the weight-gradient partial sums), grown on demand and
-// kept until the process exits.  Calls that overlap on one device share it, as they
-// share the error flag: the calls synchronize their stream before returning.
+// copy of the A source and the partial sums), grown on demand and kept until the process
+// exits.  A call holds its device's lock from here until its stream is synchronized, so
+// that calls from several threads or streams take the scratch in turn.
 struct Scratch {
+    std::mutex busy;
     int *err = nullptr;               // page-locked host memory: read after the call's synchronisation, no copy
     unsigned char *bpack = nullptr;   // 27 x 512 bytes
     __nv_bfloat16 *pad = nullptr;     // [(nz + 2)(ny + 2)(nx + 2)][16]
@@ -529,13 +530,12 @@ struct Scratch {
 
 size_t pad_bytes(const Grid &g) { return size_t(g.nz + 2) * (g.ny + 2) * (g.nx + 2) * kC * sizeof(__nv_bfloat16); }
 
-int scratch(int dev, size_t part_bytes, size_t padded_bytes, Scratch &out)
+int scratch(int dev, size_t part_bytes, size_t padded_bytes, std::unique_lock<std::mutex> &lock, Scratch *&out)
 {
-    static std::mutex mu;
     static Scratch per[64];
     if (dev < 0 || dev >= 64) return HRN_EARG;
-    std::lock_guard<std::mutex> lock(mu);
     Scratch &s = per[dev];
+    lock = std::unique_lock<std::mutex>(s.busy);
     if (!s.err) {
         void *h = nullptr;
         if (cudaHostAlloc(&h, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) != cudaSuccess) return HRN_EOOM;
@@ -558,19 +558,19 @@ int scratch(int dev, size_t part_bytes, size_t padded_bytes, Scratch &out)
         if (cudaMalloc(&s.part, part_bytes) != cudaSuccess) return HRN_EOOM;
         s.part_bytes = part_bytes;
     }
-    out = s;
+    out = &s;
     return HRN_OK;
 }
 
-int check_err(const Scratch &s, cudaStream_t st)
+// The end of a call: its launches are done (also after a failed one) and their errors known.
+int check_err(Scratch &s, cudaStream_t st)
 {
-    if (cudaStreamSynchronize(st) != cudaSuccess) return HRN_ECUDA;
+    const bool launched = cudaGetLastError() == cudaSuccess;
+    const bool done = cudaStreamSynchronize(st) == cudaSuccess;
     volatile int *e = s.err;
-    if (*e) {
-        *e = 0;
-        return HRN_ECUDA;
-    }
-    return HRN_OK;
+    const bool timed_out = *e != 0;
+    *e = 0;
+    return launched && done && !timed_out ? HRN_OK : HRN_ECUDA;
 }
 
 template <bool GRAD>
@@ -595,8 +595,10 @@ extern "C" int hrn_cnn_conv3d_forward(int32_t cin, int32_t cout, int32_t nz, int
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return HRN_ECUDA;
     const Grid g{nz, ny, nx};
-    Scratch s;
-    if (int rc = scratch(dev, 0, pad_bytes(g), s)) return rc;
+    std::unique_lock<std::mutex> lock;
+    Scratch *sp = nullptr;
+    if (int rc = scratch(dev, 0, pad_bytes(g), lock, sp)) return rc;
+    Scratch &s = *sp;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int np = (nz + 2) * (ny + 2) * (nx + 2);
     set_smem_once<false>();
@@ -605,7 +607,6 @@ extern "C" int hrn_cnn_conv3d_forward(int32_t cin, int32_t cout, int32_t nz, int
                                                           s.bpack, s.pad);
     hrn::chain_start(k_conv_band<false>, (np + kM - 1) / kM, kThreads, kConvSmem, st, true, cin, cout, g, s.pad, s.bpack, bias,
                      relu, y, s.err);
-    if (cudaGetLastError() != cudaSuccess) return HRN_ECUDA;
     return check_err(s, st);
 }
 
@@ -620,8 +621,10 @@ extern "C" int hrn_cnn_conv3d_backward(int32_t cin, int32_t cout, int32_t nz, in
     const Grid g{nz, ny, nx};
     const int V = g.size();
     const int nround = wgrad_rounds(V), nchunk = (V + nround * kWgVox - 1) / (nround * kWgVox);
-    Scratch s;
-    if (int rc = scratch(dev, size_t(nchunk) * 4 * kM * kC * sizeof(float), gx ? pad_bytes(g) : 0, s)) return rc;
+    std::unique_lock<std::mutex> lock;
+    Scratch *sp = nullptr;
+    if (int rc = scratch(dev, size_t(nchunk) * 4 * kM * kC * sizeof(float), gx ? pad_bytes(g) : 0, lock, sp)) return rc;
+    Scratch &s = *sp;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const __nv_bfloat16 *yb = static_cast<const __nv_bfloat16 *>(y);
     if (gx) {
@@ -638,6 +641,5 @@ extern "C" int hrn_cnn_conv3d_backward(int32_t cin, int32_t cout, int32_t nz, in
     const int nb = std::min((V + kBThreads / 4 - 1) / (kBThreads / 4), kBBlocks);
     k_conv_bias_part<<<nb, kBThreads, 0, st>>>(g, gy, yb, relu, s.bpart);
     k_conv_sum<<<kSumBlocks + 1, kSumThreads, 0, st>>>(cin, cout, nchunk, s.part, gw, nb, s.bpart, gb);
-    if (cudaGetLastError() != cudaSuccess) return HRN_ECUDA;
     return check_err(s, st);
 }

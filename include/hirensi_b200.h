@@ -326,8 +326,9 @@ int hrn_pseudo_hessian(hrn_ctx *ctx, double *d_h_lambda, double *d_h_mu);
  * 2^30.  All pointers are device pointers; stream is a cudaStream_t or NULL.  Returns
  * once the layer has run (the kernels' error flag is read back).  The layers keep a
  * per-device scratch (the packed weights, a copy of the input with a one-voxel zero
- * border, weight-gradient partial sums), allocated when a larger grid first needs it
- * and shared by all calls on that device: calls that overlap on one device race on it. */
+ * border, partial sums of the gradients), allocated when a larger grid first needs it
+ * and shared by all calls on that device, which take it in turn: a call from another
+ * host thread waits until the one before has returned. */
 int hrn_cnn_conv3d_forward(int32_t cin, int32_t cout, int32_t nz, int32_t ny, int32_t nx, const void *x,
                            const void *w, const float *bias, int32_t relu, void *y, void *stream);
 /* Gradients of that layer from gy = dL/dy (FP32 [nz][ny][nx][16]): gx = dL/dx (FP32
