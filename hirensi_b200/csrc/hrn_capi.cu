@@ -180,6 +180,23 @@ static int set_mass(hrn_ctx *c, const double *diag_m, bool device_src)
     return 0;
 }
 
+// A list that is refused is dropped, so that no later call reads equations out of range
+// or tables of another length.
+static int refuse_history(hrn_ctx *c, const char *why)
+{
+    c->nstore = 0;
+    c->h_store_eq.clear();
+    return set_error(c, HRN_EARG, why);
+}
+static int refuse_shots(hrn_ctx *c, int code, const char *why)
+{
+    c->nshot = 0;
+    c->h_src_eq.clear();
+    c->h_src_b.clear();
+    c->have_forward = false;
+    return set_error(c, code, why);
+}
+
 // Per-row slot map for the history.
 static int upload_store_pos(hrn_ctx *c)
 {
@@ -187,8 +204,8 @@ static int upload_store_pos(hrn_ctx *c)
     std::vector<int32_t> sp(size_t(c->neq), -1);
     for (int p = 0; p < c->nstore; ++p) {
         const int32_t e = c->h_store_eq[p];
-        if (e < 0 || e >= c->neq) return set_error(c, HRN_EARG, "history equation out of range");
-        if (sp[e] >= 0) return set_error(c, HRN_EARG, "history equation listed twice");
+        if (e < 0 || e >= c->neq) return refuse_history(c, "history equation out of range");
+        if (sp[e] >= 0) return refuse_history(c, "history equation listed twice");
         sp[e] = p;
     }
     HRN_CUDA(c, c->d_store_pos.alloc(sp.size() * 4));
@@ -204,7 +221,7 @@ static int upload_sources(hrn_ctx *c)
     const int S = c->nshot;
     std::map<int32_t, int> slot_of;
     for (int32_t e : c->h_src_eq) {
-        if (e < 0 || e >= c->neq) return set_error(c, HRN_EARG, "source equation out of range");
+        if (e < 0 || e >= c->neq) return refuse_shots(c, HRN_EARG, "source equation out of range");
         slot_of.emplace(e, 0);
     }
     int k = 0;
@@ -230,6 +247,18 @@ static int upload_sources(hrn_ctx *c)
     return 0;
 }
 
+static int upload_receivers(hrn_ctx *c);
+static int refuse_receivers(hrn_ctx *c, const char *why)
+{
+    c->nrec3 = 0;
+    c->h_eqdis.clear();
+    c->h_eqdis_map.clear();
+    c->h_rec_mask.clear();
+    c->have_data = false;
+    if (int rc = upload_receivers(c)) return rc;
+    return set_error(c, HRN_EARG, why);
+}
+
 static int upload_receivers(hrn_ctx *c)
 {
     if (c->neq == 0 || c->nshot == 0 || c->nrec3 == 0) {
@@ -244,8 +273,8 @@ static int upload_receivers(hrn_ctx *c)
     std::map<int32_t, std::vector<int32_t>> lists;
     for (int q = 0; q < c->nrec3; ++q) {
         const int32_t e = c->h_eqdis[q];
-        if (e < 0 || e >= c->neq) return set_error(c, HRN_EARG, "receiver equation out of range");
-        if (c->h_eqdis_map[q] < 0 || c->h_eqdis_map[q] >= c->nstore) return set_error(c, HRN_EARG, "receiver history position out of range");
+        if (e < 0 || e >= c->neq) return refuse_receivers(c, "receiver equation out of range");
+        if (c->h_eqdis_map[q] < 0 || c->h_eqdis_map[q] >= c->nstore) return refuse_receivers(c, "receiver history position out of range");
         lists[e].push_back(q);
     }
     std::vector<int32_t> ptr(1, 0), ql, seq;
@@ -314,10 +343,9 @@ static int check_ready(hrn_ctx *c, bool need_mesh)
 // (Re)bind everything that depends on neq once an operator exists.
 static int rebind(hrn_ctx *c)
 {
-    if (int rc = upload_store_pos(c)) return rc;
-    if (int rc = upload_sources(c)) return rc;
-    if (int rc = upload_receivers(c)) return rc;
-    return 0;
+    // all three, also past a refused list: setting that list again completes the problem
+    const int h = upload_store_pos(c), s = upload_sources(c), r = upload_receivers(c);
+    return h ? h : (s ? s : r);
 }
 
 }  // namespace hrn
@@ -668,7 +696,7 @@ int hrn_set_shots(hrn_ctx *c, int32_t nshot, int32_t nstep, double dt, int32_t n
     c->h_rec_mask.clear();
     c->have_data = false;
     for (double v : c->h_ftab)
-        if (!std::isfinite(v)) return set_error(c, HRN_ENAN, "non-finite time function sample");
+        if (!std::isfinite(v)) return refuse_shots(c, HRN_ENAN, "non-finite time function sample");
     c->have_forward = false;
     cudaSetDevice(c->device);
     HRN_CUDA(c, c->d_mis_terms.alloc(size_t(nshot) * (nstep + 1) * 8));

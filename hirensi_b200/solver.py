@@ -201,6 +201,7 @@ class Solver:
 
     def set_receivers(self, eqdis, eqdis_map):
         e, m = i32(eqdis), i32(eqdis_map)
+        self.nrec3 = 0   # a refused list is dropped
         self._check(self._L.hrn_set_receivers(self.h, e.size, iptr(e), iptr(m)))
         self.nrec3 = e.size
 

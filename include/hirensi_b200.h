@@ -115,6 +115,8 @@ int hrn_assemble_face_force(hrn_ctx *ctx, const int32_t *nface, double *b);
 int hrn_set_shots_face_force(hrn_ctx *ctx, int32_t nshot, int32_t nstep, double dt, const double *ftab);
 
 /* ---- problem description --------------------------------------------------- */
+/* A history, source or receiver list that is refused (by its setter or, if it was set
+ * before the operator, by the call that gives one) is dropped. */
 
 /* History equations U_Store_Numbers_Global (S3/PIC_Inversion_Data_Structure.F90:255-300). */
 int hrn_set_history(hrn_ctx *ctx, int32_t nstore, const int32_t *store_eq);
