@@ -340,6 +340,19 @@ __global__ void k_src_adj(int n, int nstep, int nstore, int nrec3, int nslot, co
 
 __constant__ int c_node_at[27];   // local node at GLL point q = 9c + 3b + a
 
+// The two scalars of a point from its physical gradients d[field][component][axis].
+__device__ __forceinline__ void grad_scalars(const double (&d)[2][3][3], int lambda_2mu, double &sl, double &sm)
+{
+    const auto &u = d[0];
+    const auto &p = d[1];
+    sl = (u[0][0] + u[1][1] + u[2][2]) * (p[0][0] + p[1][1] + p[2][2]);
+    const double cross = (p[0][1] + p[1][0]) * (u[0][1] + u[1][0]) + (p[0][2] + p[2][0]) * (u[0][2] + u[2][0]) +
+                         (p[2][1] + p[1][2]) * (u[2][1] + u[1][2]);
+    if (!lambda_2mu) sm = 2.0 * (u[0][0] * p[0][0] + u[1][1] * p[1][1] + u[2][2] * p[2][2]) + cross;
+    else
+        sm = -2.0 * (p[0][0] * (u[1][1] + u[2][2]) + p[1][1] * (u[0][0] + u[2][2]) + p[2][2] * (u[0][0] + u[1][1])) + cross;
+}
+
 // Elements and threads of a block: one thread per (element, point, shot).
 template <int S>
 constexpr int grad_elems() { return S >= 6 ? 1 : (S == 5 ? 2 : (S == 3 ? 3 : 8 / S)); }
@@ -347,8 +360,8 @@ constexpr int grad_elems() { return S >= 6 ? 1 : (S == 5 ? 2 : (S == 3 ? 3 : 8 /
 // Thread (element, point, shot): both fields' values of the block's elements go to shared
 // memory once, already in FP64, as [field][component][point][shot]; each thread takes the
 // two other points of its three lines from there, and the shots of a point are added in
-// order at the end.  One thread per point over all shots converted every value again for
-// each of its uses (108 a point and shot, at a sixteenth of the FP32 rate): 330 us a step
+// a fixed order at the end.  One thread per point over all shots converted every value again
+// for each of its uses (108 a point and shot, at a sixteenth of the FP32 rate): 330 us a step
 // for 32000 elements and 8 FP32 shots, 186 here.  BOX: DJI is diagonal.
 template <typename T, int S, int BOX>
 __global__ void __launch_bounds__(grad_elems<S>() * 27 * S)
@@ -412,15 +425,8 @@ k_gradient(int nel_rd, const int32_t *__restrict__ rd_store, const double *__res
                     for (int k = 0; k < 3; ++k) d[f][c][k] = x * J[k] + y * J[3 + k] + z * J[6 + k];
                 }
         }
-        const auto &u = d[0];
-        const auto &p = d[1];
-        const double sl = (u[0][0] + u[1][1] + u[2][2]) * (p[0][0] + p[1][1] + p[2][2]);
-        const double cross = (p[0][1] + p[1][0]) * (u[0][1] + u[1][0]) + (p[0][2] + p[2][0]) * (u[0][2] + u[2][0]) +
-                             (p[2][1] + p[1][2]) * (u[2][1] + u[1][2]);
-        double sm;
-        if (!lambda_2mu) sm = 2.0 * (u[0][0] * p[0][0] + u[1][1] * p[1][1] + u[2][2] * p[2][2]) + cross;
-        else
-            sm = -2.0 * (p[0][0] * (u[1][1] + u[2][2]) + p[1][1] * (u[0][0] + u[2][2]) + p[2][2] * (u[0][0] + u[1][1])) + cross;
+        double sl, sm;
+        grad_scalars(d, lambda_2mu, sl, sm);
         double fac0 = gm[9];
         if constexpr (BOX != 0) {   // GLL weights 1/3, 4/3, 1/3: the centre's is 64/27
             const int mids = (qm[0] == 1) + (qm[1] == 1) + (qm[2] == 1);
@@ -457,6 +463,79 @@ k_gradient(int nel_rd, const int32_t *__restrict__ rd_store, const double *__res
         g_lam[size_t(e) * 27 + q] += tl;
         g_mu[size_t(e) * 27 + q] += tm;
     }
+}
+
+// Thread (element, point) over all shots, the values in shared memory as
+// [field][component][element][shot][point], converted once.  A point's geometry is read
+// once and its shots are added in its thread, where the kernel above reads it once a shot,
+// leaves 5 to 16 % of the lanes idle and meets at two more barriers if the shots of a
+// point do not fill a power of two.  See grad_by_point for the measured sides.
+constexpr int kGradPtElems = 4, kGradPtThreads = 128;
+
+template <typename T, int S, int BOX>
+__global__ void __launch_bounds__(kGradPtThreads)
+k_gradient_points(int nel_rd, const int32_t *__restrict__ rd_store, const double *__restrict__ geom, const T *__restrict__ hist_n,
+                  const T *__restrict__ x2, const int32_t *__restrict__ store_eq, double *__restrict__ g_lam,
+                  double *__restrict__ g_mu, double dt, int lambda_2mu)   // g_lam, g_mu: [nel_rd][27] point slots
+{
+    constexpr int E = kGradPtElems;
+    __shared__ double sh[2][3][E][S][27];
+    const int e0 = blockIdx.x * E;
+    for (int i = threadIdx.x; i < E * 27 * S; i += kGradPtThreads) {   // consecutive threads: a node's shots
+        const int s = i % S, q = i / S % 27, le = i / (27 * S);
+        if (e0 + le >= nel_rd) break;
+        const int sn = rd_store[size_t(e0 + le) * 27 + c_node_at[q]];
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            const size_t pos = 3 * size_t(sn) + c;
+            sh[0][c][le][s][q] = double(hist_n[pos * S + s]);
+            sh[1][c][le][s][q] = double(x2[size_t(store_eq[pos]) * S + s]);
+        }
+    }
+    __syncthreads();
+    const int q = threadIdx.x % 27, le = threadIdx.x / 27, e = e0 + le;
+    if (le >= E || e >= nel_rd) return;
+    const int qm[3] = {q % 3, (q / 3) % 3, q / 9};
+    constexpr int str[3] = {1, 3, 9};
+    const double *gq = geom + (size_t(e) * 27 + q) * 10;
+    const double *gm = BOX ? geom + (size_t(e) * 27 + 13) * 10 : gq;   // a box's centre point stands for all of its points
+    double J[9], w[3][3];   // DJI; l_b'(xi_a) of the 3-point GLL basis (times DJI of a box)
+    int at[3];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) J[k] = gm[k];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+        const double j = BOX ? J[4 * m] : 1.0;
+        at[m] = q - qm[m] * str[m];
+        w[m][0] = j * (qm[m] == 0 ? -1.5 : (qm[m] == 1 ? -0.5 : 0.5));
+        w[m][1] = j * (qm[m] == 0 ? 2.0 : (qm[m] == 1 ? 0.0 : -2.0));
+        w[m][2] = j * (qm[m] == 0 ? -0.5 : (qm[m] == 1 ? 0.5 : 1.5));
+    }
+    double tl = 0.0, tm = 0.0;
+    for (int s = 0; s < S; ++s) {
+        double d[2][3][3];
+#pragma unroll
+        for (int f = 0; f < 2; ++f)
+#pragma unroll
+            for (int c = 0; c < 3; ++c) {
+#pragma unroll
+                for (int m = 0; m < 3; ++m) {
+                    const double *v = sh[f][c][le][s] + at[m];
+                    d[f][c][m] = fma(w[m][2], v[2 * str[m]], fma(w[m][1], v[str[m]], w[m][0] * v[0]));
+                }
+                if constexpr (BOX == 0) {   // physical gradients: d/dx_k = sum_m DJI(m,k) d/dxi_m
+                    const double x = d[f][c][0], y = d[f][c][1], z = d[f][c][2];
+#pragma unroll
+                    for (int k = 0; k < 3; ++k) d[f][c][k] = x * J[k] + y * J[3 + k] + z * J[6 + k];
+                }
+            }
+        double sl, sm;
+        grad_scalars(d, lambda_2mu, sl, sm);
+        tl += sl;
+        tm += sm;
+    }
+    g_lam[size_t(e) * 27 + q] += (tl * gq[9]) * dt;
+    g_mu[size_t(e) * 27 + q] += (tm * gq[9]) * dt;
 }
 
 // Node sums of the gradient slots in a fixed order (ascending element, then point),
@@ -841,20 +920,45 @@ static int build_rd_store(hrn_ctx *c)
     return 0;
 }
 
+// Which gradient kernel: one thread per point for one shot, and for shot counts that are not
+// a power of two from two blocks an SM up.  us a launch, per (point, shot) / per point, boxes
+// (general elements in brackets):
+//   16384 elements, FP32: 1 shot 19.0 / 18.8 (24.5 / 22.9), 3 shots 41.3 / 37.2 (49.5 / 42.4),
+//     5 shots 69.1 / 54.0 (72.1 / 59.8), 6 shots 73.2 / 72.0 (91.1 / 76.1), 7 shots 78.2 / 72.2
+//     (92.5 / 78.2), 8 shots 84.4 / 87.3 (95.1 / 90.6)
+//   16384 elements, FP64: 5 shots 76.1 / 59.8 (79.1 / 66.5), 7 shots 84.3 / 80.3 (104.9 / 86.4)
+//   2048 elements, FP64: 3 shots 10.4 / 10.3 (12.2 / 10.4), 7 shots 15.5 / 15.5 (18.5 / 17.4)
+//   360 elements, FP64: 1 shot 5.4 / 4.4 (5.6 / 4.2), 5 shots 6.2 / 8.3, 7 shots 6.2 / 10.3
+template <int S>
+static bool grad_by_point(const hrn_ctx *c)
+{
+    if constexpr ((S & (S - 1)) != 0) return c->nel_rd >= 2 * kGradPtElems * c->num_sms;
+    return S == 1;
+}
+
 // The correlation of one history row with one state on stream st: x2 [row][S] read
 // through rows [nstore].
 template <typename T, int S>
 static void launch_gradient(hrn_ctx *c, const T *u_n, const T *x2, const int32_t *rows, int lambda_2mu, cudaStream_t st)
 {
-    constexpr int E = grad_elems<S>();
-    const int blocks = (c->nel_rd + E - 1) / E;
     double *gsl = c->d_gslot.as<double>(), *gsm = gsl + size_t(c->nel_rd) * 27;
-    auto go = [&](auto kern) {
-        kern<<<blocks, E * 27 * S, 0, st>>>(c->nel_rd, c->d_rd_store.as<int32_t>(), c->d_rd_geom.as<double>(), u_n, x2, rows, gsl, gsm,
-                                            c->dt, lambda_2mu);
+    auto go = [&](auto kern, int elems, int threads) {
+        kern<<<(c->nel_rd + elems - 1) / elems, threads, 0, st>>>(c->nel_rd, c->d_rd_store.as<int32_t>(), c->d_rd_geom.as<double>(),
+                                                                  u_n, x2, rows, gsl, gsm, c->dt, lambda_2mu);
     };
-    if (c->rd_box) go(k_gradient<T, S, 1>);
-    else go(k_gradient<T, S, 0>);
+    constexpr int E = grad_elems<S>();
+    if constexpr (S == 1 || (S & (S - 1)) != 0) {
+        if (grad_by_point<S>(c)) {
+            if (c->rd_box) go(k_gradient_points<T, S, 1>, kGradPtElems, kGradPtThreads);
+            else go(k_gradient_points<T, S, 0>, kGradPtElems, kGradPtThreads);
+            ++c->launches;
+            return;
+        }
+    }
+    if constexpr (S > 1) {
+        if (c->rd_box) go(k_gradient<T, S, 1>, E, E * 27 * S);
+        else go(k_gradient<T, S, 0>, E, E * 27 * S);
+    }
     ++c->launches;
 }
 
