@@ -508,6 +508,7 @@ int hrn_set_mesh(hrn_ctx *c, int32_t nj, int32_t nel, int32_t neq, const double 
     if (is_line_variant(c->lanes_f)) c->lanes_f = 0;   // the new mesh may not suit the line operator: tune again
     if (is_line_variant(c->lanes_a)) c->lanes_a = 0;
     c->op_from_mesh = false;
+    if (nj != c->nj) c->lbfgs_m = 0;   // the L-BFGS vectors have another length
     c->nj = nj;
     c->nel = nel;
     c->neq = neq;

@@ -38,3 +38,35 @@ def test_elements_in_another_order(gpu_lib, matrix_free):
             out.append([s.diag_m(), s.traces()] + ops)
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+def test_lbfgs_memory_of_another_mesh(gpu_lib):
+    """The memory is sized for the mesh it was set up on: a direction on a larger one is refused."""
+    import torch
+    from hirensi_b200.capi import HrnError
+    from hirensi_b200.inversion import DeviceBackend
+    from hirensi_b200.mesh import box_mesh
+    from hirensi_b200.solver import Solver
+    small, large = box_mesh(1, 1, 1, 2.5, 1), box_mesh(3, 2, 2, 2.5, 1)
+
+    def vectors(mesh):
+        v = [torch.full((mesh.nj,), float(k), dtype=torch.float64, device="cuda") for k in range(1, 12)]
+        torch.cuda.synchronize()
+        return v
+
+    with Solver("fp64") as s:
+        v = vectors(small)
+        for again in range(2):   # set again with as many nodes: the memory stays
+            s.set_mesh(small, RHO)
+            back = DeviceBackend(s, small)
+            if not again:
+                back.lbfgs_setup(3, v[0])
+            back.lbfgs_direction(2 + again, 1, *v[:10])
+        w = vectors(large)
+        s.set_mesh(large, RHO)
+        back = DeviceBackend(s, large)
+        with pytest.raises(HrnError):
+            back.lbfgs_direction(4, 1, *w[:10])
+        back.lbfgs_setup(3, w[0])
+        back.lbfgs_direction(2, 1, *w[:10])
+        torch.cuda.synchronize()
