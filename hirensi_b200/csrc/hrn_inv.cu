@@ -528,6 +528,7 @@ int hrn_lbfgs_direction(hrn_ctx *c, int32_t iter, int32_t iter_begin, const doub
 {
     if (!c || !g_l || !g_m || !p_l || !p_m) return HRN_EARG;
     if (c->lbfgs_m < 1) return set_error(c, HRN_ESTATE, "call hrn_lbfgs_setup first");
+    if (iter < iter_begin) return set_error(c, HRN_EARG, "iter lies before iter_begin");   // no such pair
     const int n = c->nj, M = c->lbfgs_m;
     if (iter == iter_begin) {   // p = -g
         if (int rc = vec_axpby(c, n, -1.0, g_l, 0.0, nullptr, p_l)) return rc;

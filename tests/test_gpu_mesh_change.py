@@ -70,3 +70,21 @@ def test_lbfgs_memory_of_another_mesh(gpu_lib):
         back.lbfgs_setup(3, w[0])
         back.lbfgs_direction(2, 1, *w[:10])
         torch.cuda.synchronize()
+
+
+def test_lbfgs_direction_before_the_first_iteration(gpu_lib):
+    """iter < iter_begin names no pair of the memory."""
+    import torch
+    from hirensi_b200.capi import HrnError
+    from hirensi_b200.inversion import DeviceBackend
+    from hirensi_b200.solver import Solver
+    mesh = tiny()["mesh"]
+    v = [torch.full((mesh.nj,), float(k), dtype=torch.float64, device="cuda") for k in range(1, 12)]
+    torch.cuda.synchronize()
+    with Solver("fp64") as s:
+        s.set_mesh(mesh, RHO)
+        back = DeviceBackend(s, mesh)
+        back.lbfgs_setup(3, v[0])
+        for it in (-1, -4, -7):
+            with pytest.raises(HrnError):
+                back.lbfgs_direction(it, 1, *v[:10])
