@@ -225,7 +225,13 @@ static int red_space(hrn_ctx *c)
     HRN_CUDA(c, c->h_red.alloc(4 * sizeof(double)));
     if (!c->d_red.p) {
         HRN_CUDA(c, c->d_red.alloc((kRedBlocks + 1) * 8));
-        HRN_CUDA(c, cudaMemsetAsync(c->d_red.p, 0, c->d_red.bytes, c->stream));
+        // zeroed now, not on a stream that may be under capture
+        cudaError_t e = cudaMemset(c->d_red.p, 0, c->d_red.bytes);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(nullptr);
+        if (e != cudaSuccess) {
+            c->d_red.release();
+            return cuda_error(c, e, "zeroing the reduction workspace");
+        }
     }
     return 0;
 }

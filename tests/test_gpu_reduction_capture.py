@@ -1,0 +1,42 @@
+"""A scalar reduction asked for while its stream is under capture is refused, as every call
+that synchronizes is, and the calls after it are not affected."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def test_first_reduction_under_capture(gpu_lib):
+    import torch
+    from hirensi_b200.solver import Solver
+    rng = np.random.default_rng(1)
+    h = rng.standard_normal(100000)
+    # freed device memory with other contents: what the workspace may be cut from
+    for _ in range(2):
+        junk = [torch.full((1 << 18,), 7.0, dtype=torch.float64, device="cuda") for _ in range(4)]
+        torch.cuda.synchronize()
+        del junk
+        torch.cuda.empty_cache()
+    x = torch.from_numpy(h).cuda()
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    out = C.c_double()
+    p = C.c_void_p(x.data_ptr())
+    rt = C.CDLL("libcudart.so.12")   # torch's, already loaded
+    handle, graph = C.c_void_p(st.cuda_stream), C.c_void_p()
+    with Solver("fp64") as s:
+        s.set_stream(st.cuda_stream)
+        assert rt.cudaStreamBeginCapture(handle, 2) == 0   # relaxed: allocations are allowed
+        rc = gpu_lib.hrn_vec_dot(s.h, x.numel(), p, p, C.byref(out))
+        rt.cudaStreamEndCapture(handle, C.byref(graph))    # the refused call has ended the capture
+        rt.cudaGetLastError()
+        assert rc != 0
+        torch.cuda.synchronize()
+        for scale in (1.0, 2.0, 3.0):
+            x.copy_(torch.from_numpy(h * scale))
+            torch.cuda.synchronize()
+            assert gpu_lib.hrn_vec_dot(s.h, x.numel(), p, p, C.byref(out)) == 0
+            ref = float(np.dot(h * scale, h * scale))
+            assert abs(out.value - ref) <= 1e-13 * ref
