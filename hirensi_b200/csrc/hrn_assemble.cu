@@ -30,6 +30,7 @@
 
 #include <algorithm>
 #include <atomic>
+#include <limits>
 #include <vector>
 
 #include "hrn_internal.h"
@@ -43,12 +44,15 @@ __device__ double a_D[3][3];                // a_D[a][b] = l_b'(xi_a)
 __device__ unsigned char a_kI[513], a_kJ[513], a_kn[513], a_kq[513][7];
 __device__ unsigned char a_eaI[189], a_eaJ[189];   // I = J first, then the pairs along xi, eta, zeta
 
+// In place of a node's first stretching factor; finite factors of either sign are the profile's.
+constexpr double kPastTop = -std::numeric_limits<double>::infinity();
+
 struct AsmArgs {
     const int32_t *elems;      // element ids of this colour
     int nel;
     const int32_t *inod, *id;
     const double *xyz, *geom, *lam, *mu, *rho, *pml;
-    const double *pmlf;         // [nj][12] stretching factors of every node (k_asm_pml), -1 in [0] past the top
+    const double *pmlf;         // [nj][12] stretching factors of every node (k_asm_pml), kPastTop in [0] past the top
     const double *pmla;         // [nj] the factor a
     // values mode
     const int32_t *rowptr;
@@ -265,12 +269,12 @@ __global__ void k_asm_mass(AsmArgs A, int pml)
         mass_rd(A, idn, A.rho[e], fac0);
         return;
     }
-    if (A.pmlf[size_t(node) * 12] < 0.0) { atomicExch(A.err, 4); return; }
+    if (A.pmlf[size_t(node) * 12] == kPastTop) { atomicExch(A.err, 4); return; }
     mass_pml(A, idn, A.rho[e], A.pmla[node], fac0);
 }
 
 // Stretching factors of every node: F1, F2, F3 of the kinds e, p, w, then b, c, d; a first
-// entry of -1 marks a node past the top face.  The element kernels take them from here: each
+// entry of kPastTop marks a node past the top face.  The element kernels take them from here: each
 // EA entry used to evaluate the whole profile again (three divisions for a value that most
 // entries then multiply by a zero derivative).
 __global__ void k_asm_pml(int nj, const double *__restrict__ xyz, const double *__restrict__ pml, double *__restrict__ out,
@@ -280,7 +284,7 @@ __global__ void k_asm_pml(int nj, const double *__restrict__ xyz, const double *
     if (j >= nj) return;
     double ab[10], *o = out + size_t(j) * 12;
     if (!pml_ab(xyz + size_t(j) * 3, pml, ab)) {
-        o[0] = -1.0;
+        o[0] = kPastTop;
         return;
     }
     o[0] = mul(ab[0], ab[1]); o[1] = mul(ab[0], ab[2]); o[2] = mul(ab[1], ab[2]);
@@ -313,7 +317,7 @@ __device__ __forceinline__ void ea_entry(const AsmArgs &A, int I, int J, int c, 
     // entries of a direction without a derivative are zero (I and J off its line)
     const double hd = (d == 3 ? (c == 0 ? h2 : h1) : d == 4 ? (c == 0 ? h3 : h1) : d == 5 ? (c == 1 ? h3 : h2)
                                                                                           : (c == 0 ? h1 : c == 1 ? h2 : h3));
-    if (F[0] < 0.0) { atomicExch(A.err, 4); return; }
+    if (F[0] == kPastTop) { atomicExch(A.err, 4); return; }
     if (hd == 0.0 && isfinite(zl) && isfinite(zm)) return;   // 0 times a non-finite modulus is not
     const RowSeg Rs = row_seg(A, sj), Ru = row_seg(A, ui);
     int at_s = -1, at_u = -1;
@@ -377,7 +381,7 @@ __device__ __forceinline__ void element_pml(const AsmArgs &A, AsmElem &S, int e,
         const bool mass = k >= 27 * 27;
         const int I = mass ? k - 27 * 27 : k / 27, f = (k % 27) / 9, dof = k % 9;
         const int q = 9 * a_ijk[I][2] + 3 * a_ijk[I][1] + a_ijk[I][0];
-        if (S.f[I * 9] < 0.0) { atomicExch(A.err, 4); continue; }
+        if (S.f[I * 9] == kPastTop) { atomicExch(A.err, 4); continue; }
         const double rho = A.rho[e], fac0 = S.g[q * 10 + 9];
         if (mass) {
             mass_pml(A, S.id + I * 9, rho, A.pmla[nd[I]], fac0);
