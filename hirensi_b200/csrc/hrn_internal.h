@@ -200,6 +200,7 @@ struct hrn_ctx {
     // line-operator stage (variants 96-98): tables of the mesh, see hrn_line.cuh
     bool have_line = false;
     int line_ok = 0;              // 1: the mesh suits it, -1: it does not
+    const char *line_why = "";    // why it does not
     int line_npn = 0, line_nup = 0, line_nun = 0;   // PML nodes; displacement nodes in the PML, all
     int line_wd = 0, line_wt = 0;
     int line_stress_src = 0, line_stress_hist = 0;

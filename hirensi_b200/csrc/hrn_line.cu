@@ -209,15 +209,16 @@ static int line_tables(hrn_ctx *c)
     // equations of a node: three displacements in a row or none, six stresses in a row or none
     std::vector<int32_t> ubase(nj), sbase(nj), pidx(nj, -1);
     c->line_ok = -1;
-    if (c->neq >= (1 << 29)) return 0;   // 32-bit offsets into [neq][8 shots]
+    auto no = [&](const char *why) { c->line_why = why; return 0; };
+    if (c->neq >= (1 << 29)) return no("more than 2^29 equations");   // 32-bit offsets into [neq][8 shots]
     for (int j = 0; j < nj; ++j) {
         const int32_t *id = c->h_id.data() + size_t(j) * 9;
         ubase[j] = id[0];
         sbase[j] = id[3];
         for (int d = 1; d < 3; ++d)
-            if (id[d] != (id[0] < 0 ? -1 : id[0] + d)) return 0;
+            if (id[d] != (id[0] < 0 ? -1 : id[0] + d)) return no("a node's displacement equations are not numbered in a row");
         for (int d = 1; d < 6; ++d)
-            if (id[3 + d] != (id[3] < 0 ? -1 : id[3] + d)) return 0;
+            if (id[3 + d] != (id[3] < 0 ? -1 : id[3] + d)) return no("a node's stress equations are not numbered in a row");
     }
     static const unsigned char ijk[27][3] = {{2, 0, 0}, {2, 2, 0}, {0, 2, 0}, {0, 0, 0}, {2, 0, 2}, {2, 2, 2}, {0, 2, 2},
                                              {0, 0, 2}, {2, 1, 0}, {1, 2, 0}, {0, 1, 0}, {1, 0, 0}, {2, 0, 1}, {2, 2, 1},
@@ -252,10 +253,10 @@ static int line_tables(hrn_ctx *c)
     std::vector<int4> unode;
     for (int j = 0; j < nj; ++j) {
         if (!(kind[j] & 1)) {
-            if (sbase[j] >= 0) return 0;   // a stress unknown outside the PML
+            if (sbase[j] >= 0) return no("a stress unknown lies outside the PML");
             continue;
         }
-        if (sbase[j] < 0) return 0;        // constrained stresses
+        if (sbase[j] < 0) return no("the stresses of a PML node are constrained");
         pidx[j] = int32_t(pnode.size());
         pnode.push_back(make_int2(j, sbase[j]));
         pn_id.push_back(j);
@@ -274,8 +275,9 @@ static int line_tables(hrn_ctx *c)
         if (pass == 0) c->line_nup = int(unode.size());
     }
     const int nun = int(unode.size()), npn = int(pnode.size());
-    if (int64_t(3) * nun + int64_t(6) * npn != c->neq) return 0;   // every equation belongs to one node
-    if (most > kLineNb || nun == 0) return 0;
+    if (int64_t(3) * nun + int64_t(6) * npn != c->neq) return no("an equation belongs to no node or to several");
+    if (most > kLineNb) return no("more than 32 elements share a node");
+    if (nun == 0) return no("no displacement is free");
     c->line_nun = nun;
     c->line_npn = npn;
     std::vector<int32_t> &row = c->line_row;
@@ -352,7 +354,8 @@ static int line_tables(hrn_ctx *c)
     int flag = 0;
     HRN_CUDA(c, cudaMemcpyAsync(&flag, bad.p, 4, cudaMemcpyDeviceToHost, c->stream));
     HRN_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (flag) return 0;   // too many nodes on the lines of one, or weights that vary along a line
+    if (flag == 1) return no("more than 32 nodes lie on the grid lines through one");
+    if (flag) return no("the PML's weights across a grid line vary along it (its elements are not aligned with the axes)");
     const int box = c->rd_box ? 1 : 0;
     const int64_t ng = int64_t(c->nel_rd_e) * (box ? 4 : 270);
     HRN_CUDA(c, c->d_line_rgeo.alloc(std::max<size_t>(size_t(ng), 1) * 8));

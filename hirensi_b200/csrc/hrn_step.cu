@@ -1107,7 +1107,7 @@ static int line_check(hrn_ctx *c)
     if (!c->op_from_mesh) return set_error(c, HRN_ESTATE, "the matrix-free variants need an operator assembled from the mesh");
     int ok = 0;
     if (int rc = line_ready(c, &ok)) return rc;
-    if (!ok) return set_error(c, HRN_EARG, "the line variants need each node's displacements and stresses numbered in a row");
+    if (!ok) return set_error(c, HRN_EARG, std::string("the line variants do not serve this mesh: ") + c->line_why);
     return 0;
 }
 
