@@ -1315,6 +1315,17 @@ static int forward_t(hrn_ctx *c)
     return 0;
 }
 
+// A stored state of the line operator (by row) in the order of the equations, three vectors.
+template <typename T, int S>
+__global__ void k_state_by_equation(int neq, const int32_t *__restrict__ row, const T *__restrict__ in, T *__restrict__ out)
+{
+    for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < int64_t(3) * neq * S; i += int64_t(gridDim.x) * blockDim.x) {
+        const int s = int(i % S), eq = int(i / S % neq);
+        const size_t vec = size_t(i / S / neq);
+        out[i] = in[(vec * neq + size_t(row[eq])) * S + s];
+    }
+}
+
 template <typename T, int S>
 static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
 {
@@ -1362,13 +1373,18 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
         if (is_gtp_variant(c->lanes_a))
             if (int rc = gtp_prepare(c, 1)) return rc;
     }
-    if (c->ckpt > 0 && is_line_variant(c->fwd_variant)) {   // the recomputed forward segments
+    // the recomputed forward segments: as they were stepped, or, where the mesh that the line
+    // operator took was replaced in the meantime, by the stored operator
+    const bool by_row = c->ckpt > 0 && is_line_variant(c->fwd_variant);
+    const bool reorder = by_row && !c->op_from_mesh && c->have_pattern;
+    const int refwd = reorder ? 41 : c->fwd_variant;
+    if (c->ckpt > 0 && is_line_variant(refwd)) {
         if (int rc = line_check(c)) return rc;
-    } else if (c->ckpt > 0 && is_elem_variant(c->fwd_variant)) {
+    } else if (c->ckpt > 0 && is_elem_variant(refwd)) {
         if (int rc = elem_ready(c)) return rc;
-    } else if (c->ckpt > 0 && is_gt_variant(c->fwd_variant)) {
+    } else if (c->ckpt > 0 && is_gt_variant(refwd)) {
         if (int rc = gt_ready(c, 0)) return rc;
-        if (is_gtp_variant(c->fwd_variant))
+        if (is_gtp_variant(refwd))
             if (int rc = gtp_prepare(c, 0)) return rc;
     }
     cudaEvent_t t0, t1;
@@ -1397,15 +1413,20 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
             if (K > 0 && (n == c->nstep || n % K == K - 1)) {
                 // recompute the forward history of steps k0 .. min(k0 + K - 1, nstep - 1) from the checkpoint
                 T *R0 = c->d_Xr.as<T>(), *R1 = R0 + 3 * vn;
-                HRN_CUDA(c, cudaMemcpyAsync(R0, c->d_ckpt.as<T>() + size_t(n / K) * 3 * vn, 3 * vn * sizeof(T),
-                                            cudaMemcpyDeviceToDevice, c->stream));
+                const T *ck = c->d_ckpt.as<T>() + size_t(n / K) * 3 * vn;
+                if (reorder) {
+                    k_state_by_equation<T, S><<<blocks_for(int64_t(3 * vn), 256), 256, 0, c->stream>>>(c->neq, c->d_line_row.as<int32_t>(), ck, R0);
+                    ++c->launches;
+                } else {
+                    HRN_CUDA(c, cudaMemcpyAsync(R0, ck, 3 * vn * sizeof(T), cudaMemcpyDeviceToDevice, c->stream));
+                }
                 const int m1 = std::min(k0 + K - 1, c->nstep - 1);
                 for (int m = k0; m <= m1; ++m) {
                     af.srcv = forward_src<T, S>(c, m);
                     af.hist = c->d_ckseg.as<T>() + size_t(m - k0) * c->nstore * S;
-                    const bool odd = ((m - k0) & 1) && !is_line_variant(c->fwd_variant);
+                    const bool odd = ((m - k0) & 1) && !is_line_variant(refwd);
                     T *Xm = odd ? R1 : R0, *Ym = odd ? R0 : R1;
-                    launch_step<T, S>(c, af, Xm, Ym, c->timing ? &tm : nullptr, c->fwd_variant, taf, 0, m == k0);
+                    launch_step<T, S>(c, af, Xm, Ym, c->timing ? &tm : nullptr, refwd, taf, 0, m == k0);
                 }
             }
             const T *u_n = K > 0 ? c->d_ckseg.as<T>() + size_t(n - k0) * c->nstore * S
@@ -1438,7 +1459,7 @@ static int adjoint_t(hrn_ctx *c, int lambda_2mu, int keep_p)
         HRN_CUDA(c, cudaGetLastError());
         return 0;
     };
-    const uint64_t sig[6] = {alloc_generation().load(), c->epoch, uint64_t(c->lanes_a) | (uint64_t(c->fwd_variant) << 32),
+    const uint64_t sig[6] = {alloc_generation().load(), c->epoch, uint64_t(c->lanes_a) | (uint64_t(refwd) << 32) | (uint64_t(reorder) << 63),
                              uint64_t(keep_p != 0), uint64_t(lambda_2mu != 0), uintptr_t(c->stream)};
     const int rc = run_loop(c, c->gadj, sig, body);
     cudaEventRecord(t1, c->stream);

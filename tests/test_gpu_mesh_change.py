@@ -88,3 +88,30 @@ def test_lbfgs_direction_before_the_first_iteration(gpu_lib):
         for it in (-1, -4, -7):
             with pytest.raises(HrnError):
                 back.lbfgs_direction(it, 1, *v[:10])
+
+
+@pytest.mark.parametrize("nshot,precision", [(1, "fp64"), (3, "fp64"), (4, "fp32")])
+def test_mesh_set_between_forward_and_adjoint(gpu_lib, nshot, precision):
+    """Checkpoints of the line operator, whose tables go with the mesh: the stored operator
+    recomputes the segments.  Bars: 1e-11 between FP64 variants, 1e-4 with FP32 stepping."""
+    from problems import rel_l2
+    from hirensi_b200.solver import Solver
+    p = tiny(nshot=nshot, nstep=30)
+    dis = 1e-6 * np.random.default_rng(3).standard_normal((nshot, len(p["eqdis"]), p["nstep"] + 1))
+    out = []
+    for again in (False, True):
+        with Solver(precision) as s:
+            s.set_mesh(p["mesh"], RHO)
+            s.assemble(p["lam"], p["mu"])
+            _shots(s, p, p["mesh"])
+            s.set_checkpointing(7)
+            s.set_variant(97, 97)
+            s.forward()
+            states = s.state(14, 0)
+            if again:
+                s.set_mesh(p["mesh"], RHO)
+                assert all(np.array_equal(a, b) for a, b in zip(states, s.state(14, 0)))
+            g = s.adjoint_gradient(dis)
+            out.append(g + s.adjoint_gradient(dis))
+    for a, b in zip(*out):
+        assert rel_l2(a, b) < (1e-11 if precision == "fp64" else 1e-4)
