@@ -340,6 +340,14 @@ static int check_ready(hrn_ctx *c, bool need_mesh)
     return 0;
 }
 
+// The matrix-free variants need an operator assembled from the mesh: without one, tune again.
+static void drop_mesh_operator(hrn_ctx *c)
+{
+    c->op_from_mesh = false;
+    if (c->lanes_f >= 90 && c->lanes_f <= 105) c->lanes_f = 0;
+    if (c->lanes_a >= 90 && c->lanes_a <= 105) c->lanes_a = 0;
+}
+
 // (Re)bind everything that depends on neq once an operator exists.
 static int rebind(hrn_ctx *c)
 {
@@ -477,9 +485,7 @@ int hrn_set_operator_csr(hrn_ctx *c, int32_t neq, const int32_t *c_ia, const int
     if (int rc = launch_scale_operator(c)) return rc;
     HRN_CUDA(c, cudaStreamSynchronize(c->stream));
     c->have_operator = true;
-    c->op_from_mesh = false;
-    if (c->lanes_f >= 90 && c->lanes_f <= 105) c->lanes_f = 0;   // matrix-free needs an assembled operator: tune again
-    if (c->lanes_a >= 90 && c->lanes_a <= 105) c->lanes_a = 0;
+    drop_mesh_operator(c);
     c->have_forward = false;
     return rebind(c);
 }
@@ -552,7 +558,12 @@ static int assemble_common(hrn_ctx *c, const double *lambda, const double *mu, b
         HRN_CUDA(c, cudaMemcpyAsync(c->d_mu.p, mu, size_t(c->nj) * 8, cudaMemcpyHostToDevice, c->stream));
     }
     const bool first = c->mf_only ? !c->have_operator : !c->have_pattern;
-    if (int rc = assemble_device(c, !c->mf_only && first)) return rc;
+    if (int rc = assemble_device(c, !c->mf_only && first)) {
+        // the stored operator is still the one before; d_lam and d_mu, which the variants
+        // without one read, are not
+        drop_mesh_operator(c);
+        return rc;
+    }
     c->have_operator = true;
     c->op_from_mesh = true;
     c->have_forward = false;
