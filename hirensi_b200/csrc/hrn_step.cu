@@ -1584,7 +1584,7 @@ static int time_stage_t(hrn_ctx *c, int adj, int nsteps, double *avg_ms)
     for (int n = 0; n < nsteps; ++n) {
         const bool odd = (n & 1) && !is_line_variant(lanes);
         T *X = odd ? X1 : X0, *Y = odd ? X0 : X1;
-        launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj, n == 0);
+        launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj, 0);   // on from the warm-up, which prepared the line operator
     }
     cudaEventRecord(e1, c->stream);
     const cudaError_t es = cudaEventSynchronize(e1);
