@@ -15,7 +15,8 @@ def test_forward_after_a_failed_reassembly(gpu_lib, variant):
     p = tiny(nshot=2, nstep=30)
     mesh = p["mesh"]
     bad = torch.from_numpy(p["lam"]).cuda()
-    bad[mesh.inod[0, 0]] = float("nan")   # entries outside the pattern of the first assembly
+    inner = int(np.nonzero(mesh.node_mat_id == 0)[0][0])
+    bad[inner] = float("nan")   # entries outside the pattern of the first assembly
     mu = torch.from_numpy(p["mu"]).cuda()
     torch.cuda.synchronize()
     with Solver("fp64") as s:
