@@ -1042,8 +1042,8 @@ static double sum_timer(hrn_ctx *c, const StageTimer &tm)
     return tot;
 }
 
-// Lanes per row for one operator: the fastest of 4, 8 and 16 over a few full
-// RK4 steps on the zero state (the traffic does not depend on the values).
+// Stage variant for one operator: the fastest of the candidates over a few full RK4 steps,
+// each from the zero state (the line variants step X in place).
 template <typename T, int S>
 static int autotune_lanes(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, const TileArgs &ta, int adj)
 {
@@ -1082,10 +1082,14 @@ static int autotune_lanes(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, const TileArgs
     }
     if (cand.empty())
         return set_error(c, HRN_EARG, "no stage variant serves this operator, shot count and precision");
+    if (cand.size() == 1) return cand[0];
+    if (adj && c->nslot_a > 0)   // not written before the first adjoint step
+        HRN_CUDA(c, cudaMemsetAsync(c->d_srcv_a.p, 0, c->d_srcv_a.bytes, c->stream));
     cudaEvent_t e0, e1;
     cudaEventCreate(&e0);
     cudaEventCreate(&e1);
     for (int lanes : cand) {
+        cudaMemsetAsync(X, 0, size_t(3) * c->neq * S * sizeof(T), c->stream);
         launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj, 1);   // warm-up
         cudaEventRecord(e0, c->stream);
         for (int r = 0; r < 3; ++r) launch_step<T, S>(c, a, X, Y, nullptr, lanes, ta, adj, 0);
