@@ -787,11 +787,16 @@ int hrn_get_state(hrn_ctx *c, int32_t step, int32_t shot, double *x1, double *x2
     HRN_CUDA(c, cudaStreamSynchronize(c->stream));
     HRN_CUDA(c, cudaMemcpy(h.data(), static_cast<const unsigned char *>(c->d_ckpt.p) + size_t(step / c->ckpt) * 3 * vn * eb,
                            h.size(), cudaMemcpyDeviceToHost));
+    std::vector<int32_t> by_eq;   // the line operator's states are stored by row
+    if (is_line_variant(c->fwd_variant)) {
+        by_eq.resize(size_t(c->neq));
+        HRN_CUDA(c, cudaMemcpy(by_eq.data(), c->d_line_row.p, by_eq.size() * 4, cudaMemcpyDeviceToHost));
+    }
     double *out[3] = {x1, x2, x3};
     for (int k = 0; k < 3; ++k) {
         if (!out[k]) continue;
         for (int i = 0; i < c->neq; ++i) {
-            const size_t row = is_line_variant(c->fwd_variant) ? size_t(c->line_row[i]) : size_t(i);
+            const size_t row = by_eq.empty() ? size_t(i) : size_t(by_eq[i]);
             const size_t at = size_t(k) * vn + row * S + size_t(shot);
             out[k][i] = c->precision == HRN_FP64 ? reinterpret_cast<const double *>(h.data())[at]
                                                  : double(reinterpret_cast<const float *>(h.data())[at]);

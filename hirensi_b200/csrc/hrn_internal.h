@@ -205,8 +205,8 @@ struct hrn_ctx {
     int line_wd = 0, line_wt = 0;
     int line_stress_src = 0, line_stress_hist = 0;
     uint64_t line_epoch = 0;      // settings epoch of the two flags and of the row lists below
-    std::vector<int32_t> line_row;               // [neq] state row of an equation
-    hrn::DevBuf d_line_row, d_line_store_row, d_line_rec_row;
+    hrn::DevBuf d_line_row;       // [neq] state row of an equation
+    hrn::DevBuf d_line_store_row, d_line_rec_row;
     hrn::DevBuf d_line_pnode, d_line_didx, d_line_dcf, d_line_pcoef;
     hrn::DevBuf d_line_unode, d_line_ucoef, d_line_uim, d_line_tidx, d_line_tcf, d_line_ridx;
     hrn::DevBuf d_line_rpt, d_line_rgeo, d_line_runode;

@@ -4,14 +4,10 @@
 // them depend on the mesh alone, so they are built once per mesh.
 #include <cuda_runtime.h>
 #include <stdint.h>
-#include <thrust/execution_policy.h>
-#include <thrust/device_ptr.h>
-#include <thrust/functional.h>
-#include <thrust/reduce.h>
+#include <cub/device/device_scan.cuh>
 
 #include <algorithm>
 #include <cmath>
-#include <vector>
 
 #include "hrn_internal.h"
 
@@ -34,15 +30,15 @@ __device__ __forceinline__ double gll_d(int a, int b)   // l_b'(xi_a)
 
 // Entries of row r of D_k (TR = 0: PML node J, columns the nodes on its lines) or of
 // D_k^T (TR = 1: displacement node I, columns the PML nodes J whose lines pass it), at
-// most w a direction (TR = 0) or a row (TR = 1).  idx == null: count them, per direction
-// into cnt[3 r + k] or per row into cnt[r]; else write them, entry u of a direction at
+// most w a direction (TR = 0) or a row (TR = 1).  idx == null: the most a direction or a
+// row has, into *most; else write them, entry u of a direction at
 // idx[(k w + u) nrow + r], of a row at idx[u nrow + r], divided by fj = F j0 of node J.
 template <typename T, int TR>
 __global__ void __launch_bounds__(kLineBuildThreads)
 k_line_entries(int nrow, const int32_t *__restrict__ nodes, const int32_t *__restrict__ nptr, const uint32_t *__restrict__ nslot,
                int nel_pml, const int32_t *__restrict__ el_node, const double *__restrict__ geom,
                const int32_t *__restrict__ target, int ntarget, const double *__restrict__ pmlw, const double *__restrict__ fj, int w,
-               int32_t *__restrict__ cnt, int32_t *__restrict__ idx, T *__restrict__ cf, int *__restrict__ bad)
+               int *most, int32_t *__restrict__ idx, T *__restrict__ cf, int *__restrict__ bad)
 {
     __shared__ int32_t s_nb[kLineNb][kLineBuildThreads];
     __shared__ double s_cf[3][kLineNb][kLineBuildThreads];
@@ -78,6 +74,9 @@ k_line_entries(int nrow, const int32_t *__restrict__ nodes, const int32_t *__res
     for (int k = 0; k < n; ++k)
         for (int x = 0; x < 3; ++x) top = fmax(top, fabs(s_cf[x][k][th]));
     int at = 0;
+    auto raise = [&]() {   // most threads find their count there
+        if (at > *static_cast<volatile int *>(most)) atomicMax(most, at);
+    };
     for (int x = 0; x < 3; ++x) {
         if (!TR) at = 0;
         for (int k = 0; k < n; ++k) {
@@ -95,9 +94,9 @@ k_line_entries(int nrow, const int32_t *__restrict__ nodes, const int32_t *__res
             }
             ++at;
         }
-        if (!idx && !TR) cnt[3 * r + x] = at;
+        if (!idx && !TR) raise();
     }
-    if (!idx && TR) cnt[r] = at;
+    if (!idx && TR) raise();
 }
 
 // Coefficient planes of the PML nodes' stress rows (disp = 0) or of the displacement
@@ -150,11 +149,15 @@ __global__ void k_line_fj(int n, const int32_t *__restrict__ ids, const int32_t 
     out[r] = F * j0;
 }
 
-// State rows of a list of equations.
-__global__ void k_line_rows(int n, const int32_t *__restrict__ row, const int32_t *__restrict__ eq, int32_t *__restrict__ out)
+// State rows of a list of equations (out may be null), and whether one is a stress row.
+__global__ void k_line_rows(int n, int first_stress, const int32_t *__restrict__ row, const int32_t *__restrict__ eq,
+                            int32_t *__restrict__ out, int *__restrict__ stress)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) out[i] = row[eq[i]];
+    if (i >= n) return;
+    const int r = row[eq[i]];
+    if (out) out[i] = r;
+    if (r >= first_stress) atomicExch(stress, 1);
 }
 
 __global__ void k_line_rgeo(int64_t n, int box, const double *__restrict__ geom, double *__restrict__ out)
@@ -176,147 +179,196 @@ static int build_entries(hrn_ctx *c, int nrow, const DevBuf &nodes, const DevBuf
 {
     *w = 0;
     if (nrow == 0) return 0;
-    DevBuf cnt;
     const size_t nc = size_t(nrow) * (TR ? 1 : 3);
-    HRN_CUDA(c, cnt.alloc(nc * 4));
-    HRN_CUDA(c, cudaMemsetAsync(cnt.p, 0, cnt.bytes, c->stream));
+    int *most = bad.as<int>() + 1;
+    HRN_CUDA(c, cudaMemsetAsync(most, 0, 4, c->stream));
     const int nb = (nrow + kLineBuildThreads - 1) / kLineBuildThreads;
     auto launch = [&](int32_t *out) {
         k_line_entries<T, TR><<<nb, kLineBuildThreads, 0, c->stream>>>(
             nrow, nodes.as<int32_t>(), c->d_nslot_ptr.as<int32_t>(), c->d_nslot.as<uint32_t>(), c->nel_pml_e,
             c->d_el_node.as<int32_t>(), c->d_el_geom.as<double>(), target.as<int32_t>(), c->line_npn, c->d_pmlw.as<double>(), fj.as<double>(), *w,
-            cnt.as<int32_t>(), out, cf.as<T>(), bad.as<int>());
+            most, out, cf.as<T>(), bad.as<int>());
         ++c->launches;
         return cudaGetLastError();
     };
     HRN_CUDA(c, launch(nullptr));
-    thrust::device_ptr<int32_t> p(cnt.as<int32_t>());
-    *w = std::max(1, thrust::reduce(thrust::cuda::par.on(c->stream), p, p + nc, 0, thrust::maximum<int32_t>()));
+    HRN_CUDA(c, cudaMemcpyAsync(w, most, 4, cudaMemcpyDeviceToHost, c->stream));
+    HRN_CUDA(c, cudaStreamSynchronize(c->stream));
+    *w = std::max(*w, 1);
     const size_t n = nc * size_t(*w);
     HRN_CUDA(c, idx.alloc(n * 4));
     HRN_CUDA(c, cf.alloc(n * sizeof(T)));
     HRN_CUDA(c, cudaMemsetAsync(idx.p, 0xff, n * 4, c->stream));   // -1: no entry
     HRN_CUDA(c, cudaMemsetAsync(cf.p, 0, n * sizeof(T), c->stream));
     HRN_CUDA(c, launch(idx.as<int32_t>()));
-    HRN_CUDA(c, cudaStreamSynchronize(c->stream));   // cnt is released here
     return 0;
 }
 
+// What the numbering of the nodes says, and the place of every node among those that the
+// tables list: flag [3][nj + 1] is 1 where a node has a record of P, a free displacement in
+// the PML, one outside of it.
+constexpr int kLineDispRow = 1, kLineStressRow = 2, kLineStressOut = 4, kLineStressFixed = 8;
+
+__global__ void k_line_nodes(int nj, const int32_t *__restrict__ id, const int32_t *__restrict__ nptr, const uint32_t *__restrict__ nslot,
+                             int nel_pml, int32_t *__restrict__ flag, int32_t *__restrict__ nrd, int *__restrict__ info)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j > nj) return;
+    int32_t in_pml = 0, rd = 0, u = 0, why = 0;
+    if (j < nj) {
+        for (int s = nptr[j]; s < nptr[j + 1]; ++s) {
+            if (int((nslot[s] & 0x7fffffffu) / 27) < nel_pml) in_pml = 1;
+            else ++rd;
+        }
+        const int32_t *e = id + size_t(j) * 9;
+        for (int d = 1; d < 3; ++d)
+            if (e[d] != (e[0] < 0 ? -1 : e[0] + d)) why |= kLineDispRow;
+        for (int d = 1; d < 6; ++d)
+            if (e[3 + d] != (e[3] < 0 ? -1 : e[3] + d)) why |= kLineStressRow;
+        if (!in_pml && e[3] >= 0) why |= kLineStressOut;
+        if (in_pml && e[3] < 0) why |= kLineStressFixed;
+        u = e[0] >= 0;
+        nrd[j] = rd;
+        if (why) atomicOr(info, why);
+        if (u) atomicMax(info + 1, rd);
+    }
+    const size_t n = size_t(nj) + 1;   // the last entry is 0: its sum is the total
+    flag[j] = in_pml;
+    flag[n + j] = u && in_pml;
+    flag[2 * n + j] = u && !in_pml;
+}
+
+// The lists, from the sums `at` of those flags (at[..][j + 1] > at[..][j] where it is 1).
+// Rows of the state: displacements [3][nun], those of the PML first, then stresses [6][npn].
+__global__ void k_line_lists(int nj, int npn, int nup, int nun, const int32_t *__restrict__ id, const int32_t *__restrict__ at,
+                             const int32_t *__restrict__ nrd, int2 *__restrict__ pnode, int4 *__restrict__ unode,
+                             int32_t *__restrict__ pn_id, int32_t *__restrict__ pn_eq, int32_t *__restrict__ un_id,
+                             int32_t *__restrict__ un_eq, int32_t *__restrict__ pidx, int32_t *__restrict__ zidx,
+                             int32_t *__restrict__ unidx, int32_t *__restrict__ row)
+{
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= nj) return;
+    const size_t n = size_t(nj) + 1;
+    const int32_t u0 = id[size_t(j) * 9], s0 = id[size_t(j) * 9 + 3];
+    const int32_t p = at[j + 1] > at[j] ? at[j] : -1;
+    const bool up = at[n + j + 1] > at[n + j], ur = at[2 * n + j + 1] > at[2 * n + j];
+    const int32_t u = up ? at[n + j] : (ur ? nup + at[2 * n + j] : -1);
+    pidx[j] = p;
+    zidx[j] = u0 < 0 ? -1 : p;   // records of Z: PML nodes whose displacements are free
+    unidx[j] = u;
+    if (p >= 0) {
+        pnode[p] = make_int2(j, s0);
+        pn_id[p] = j;
+        pn_eq[p] = s0;
+        for (int d = 0; d < 6; ++d) row[s0 + d] = 3 * nun + d * npn + p;
+    }
+    if (u >= 0) {
+        unode[u] = make_int4(u0, p, nrd[j], 0);
+        un_id[u] = j;
+        un_eq[u] = u0;
+        for (int d = 0; d < 3; ++d) row[u0 + d] = d * nun + u;
+    }
+}
+
+// Regular-domain contributions of every displacement node, in ascending element order.
+__global__ void k_line_ridx(int nun, int nrd, int nel_pml, const int32_t *__restrict__ un_id, const int32_t *__restrict__ nptr,
+                            const uint32_t *__restrict__ nslot, int32_t *__restrict__ ridx)
+{
+    const int u = blockIdx.x * blockDim.x + threadIdx.x;
+    if (u >= nun) return;
+    int k = 0;
+    for (int s = nptr[un_id[u]]; s < nptr[un_id[u] + 1]; ++s) {
+        const uint32_t sl = nslot[s] & 0x7fffffffu;
+        const int p = int(sl / 27), q = int(sl % 27);
+        if (p >= nel_pml) ridx[size_t(k++) * nun + u] = 3 * nrd * q + (p - nel_pml);
+    }
+}
+
+// Nodes of the regular-domain elements' points, by element and by point.
+__global__ void k_line_points(int nrd, const int32_t *__restrict__ el_node, const int32_t *__restrict__ unidx, int2 *__restrict__ rpt,
+                              int32_t *__restrict__ runode)
+{
+    const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+    if (t >= int64_t(nrd) * 27) return;
+    const int e = int(t / 27), q = int(t % 27), node = el_node[t], u = unidx[node];
+    rpt[t] = make_int2(node, u);
+    runode[size_t(q) * nrd + e] = u;
+}
+
+// The tables are made on the device, from the element and node lists of elem_prepare: host
+// loops over the nodes and element points took 190 ms of the first solve on a mesh of 7.4
+// million equations, more than the timing of the element variants that they spare (first
+// forward of one FP32 shot, matrix-free, ten steps: 206 ms with those, 340 with the loops, 175
+// here; 309 thousand equations 8.3, 11.1 and 9.2).
 template <typename T>
 static int line_tables(hrn_ctx *c)
 {
-    const int nj = c->nj;
-    // equations of a node: three displacements in a row or none, six stresses in a row or none
-    std::vector<int32_t> ubase(nj), sbase(nj), pidx(nj, -1);
+    const int nj = c->nj, nrd = c->nel_rd_e;
     c->line_ok = -1;
     auto no = [&](const char *why) { c->line_why = why; return 0; };
     if (c->neq >= (1 << 29)) return no("more than 2^29 equations");   // 32-bit offsets into [neq][8 shots]
-    for (int j = 0; j < nj; ++j) {
-        const int32_t *id = c->h_id.data() + size_t(j) * 9;
-        ubase[j] = id[0];
-        sbase[j] = id[3];
-        for (int d = 1; d < 3; ++d)
-            if (id[d] != (id[0] < 0 ? -1 : id[0] + d)) return no("a node's displacement equations are not numbered in a row");
-        for (int d = 1; d < 6; ++d)
-            if (id[3 + d] != (id[3] < 0 ? -1 : id[3] + d)) return no("a node's stress equations are not numbered in a row");
+    DevBuf d_flag, d_nrd, d_info, d_pn, d_pe, d_un, d_ue, d_zi, d_pi, d_ui, d_fj, bad;
+    const size_t n1 = size_t(nj) + 1;
+    HRN_CUDA(c, d_flag.alloc(3 * n1 * 4));
+    HRN_CUDA(c, d_nrd.alloc(size_t(nj) * 4));
+    HRN_CUDA(c, d_info.alloc(8));
+    HRN_CUDA(c, cudaMemsetAsync(d_info.p, 0, 8, c->stream));
+    int32_t *flag = d_flag.as<int32_t>();
+    k_line_nodes<<<(nj + 256) / 256, 256, 0, c->stream>>>(nj, c->d_id.as<int32_t>(), c->d_nslot_ptr.as<int32_t>(),
+                                                          c->d_nslot.as<uint32_t>(), c->nel_pml_e, flag, d_nrd.as<int32_t>(), d_info.as<int>());
+    ++c->launches;
+    HRN_CUDA(c, cudaGetLastError());
+    int info[2], total[3];
+    DevBuf d_tmp;   // of the scans, which throw nothing
+    size_t tmp = 0;
+    HRN_CUDA(c, cub::DeviceScan::ExclusiveSum(nullptr, tmp, flag, flag, int(n1), c->stream));
+    HRN_CUDA(c, d_tmp.alloc(std::max<size_t>(tmp, 16)));
+    for (int k = 0; k < 3; ++k) {
+        HRN_CUDA(c, cub::DeviceScan::ExclusiveSum(d_tmp.p, tmp, flag + k * n1, flag + k * n1, int(n1), c->stream));
+        HRN_CUDA(c, cudaMemcpyAsync(&total[k], flag + k * n1 + nj, 4, cudaMemcpyDeviceToHost, c->stream));
     }
-    static const unsigned char ijk[27][3] = {{2, 0, 0}, {2, 2, 0}, {0, 2, 0}, {0, 0, 0}, {2, 0, 2}, {2, 2, 2}, {0, 2, 2},
-                                             {0, 0, 2}, {2, 1, 0}, {1, 2, 0}, {0, 1, 0}, {1, 0, 0}, {2, 0, 1}, {2, 2, 1},
-                                             {0, 2, 1}, {0, 0, 1}, {2, 1, 2}, {1, 2, 2}, {0, 1, 2}, {1, 0, 2}, {1, 1, 0},
-                                             {2, 1, 1}, {1, 2, 1}, {0, 1, 1}, {1, 0, 1}, {1, 1, 2}, {1, 1, 1}};
-    unsigned char node_at[27];
-    for (int i = 0; i < 27; ++i) node_at[9 * ijk[i][2] + 3 * ijk[i][1] + ijk[i][0]] = (unsigned char)i;
-    std::vector<unsigned char> kind(nj, 0);   // 1: in the PML, 2: in the regular domain
-    std::vector<int32_t> rptr(size_t(nj) + 1, 0);
-    for (int e = 0; e < c->nel; ++e)
-        for (int i = 0; i < 27; ++i) {
-            const int j = c->h_inod[size_t(e) * 27 + i];
-            kind[j] |= (unsigned char)c->h_mtel[e] == 2 ? 1 : 2;
-            if (c->h_mtel[e] == 1) rptr[j + 1]++;
-        }
-    for (int j = 0; j < nj; ++j) rptr[j + 1] += rptr[j];
-    std::vector<int32_t> rlist(std::max<size_t>(size_t(rptr[nj]), 1), 0), pos(rptr.begin(), rptr.end() - 1);
-    std::vector<int2> rpt(std::max<size_t>(size_t(c->nel_rd_e) * 27, 1));
-    int k = 0;
-    for (int e = 0; e < c->nel; ++e) {
-        if (c->h_mtel[e] != 1) continue;
-        for (int q = 0; q < 27; ++q) {
-            const int j = c->h_inod[size_t(e) * 27 + node_at[q]];
-            rpt[size_t(k) * 27 + q] = make_int2(j, -1);
-            rlist[pos[j]++] = k * 27 + q;
-        }
-        ++k;
-    }
-    // rows of the state: displacements [3][nun], then stresses [6][npn]
-    std::vector<int2> pnode;
-    std::vector<int32_t> pn_id, pn_eq, un_id, un_eq, unidx(nj, -1);
-    std::vector<int4> unode;
-    for (int j = 0; j < nj; ++j) {
-        if (!(kind[j] & 1)) {
-            if (sbase[j] >= 0) return no("a stress unknown lies outside the PML");
-            continue;
-        }
-        if (sbase[j] < 0) return no("the stresses of a PML node are constrained");
-        pidx[j] = int32_t(pnode.size());
-        pnode.push_back(make_int2(j, sbase[j]));
-        pn_id.push_back(j);
-        pn_eq.push_back(sbase[j]);
-    }
-    int most = 0;
-    for (int pass = 0; pass < 2; ++pass) {
-        for (int j = 0; j < nj; ++j) {
-            if (ubase[j] < 0 || ((kind[j] & 1) != 0) != (pass == 0)) continue;
-            unidx[j] = int32_t(unode.size());
-            unode.push_back(make_int4(ubase[j], pidx[j], rptr[j + 1] - rptr[j], 0));
-            un_id.push_back(j);
-            un_eq.push_back(ubase[j]);
-            most = std::max(most, rptr[j + 1] - rptr[j]);
-        }
-        if (pass == 0) c->line_nup = int(unode.size());
-    }
-    const int nun = int(unode.size()), npn = int(pnode.size());
+    HRN_CUDA(c, cudaMemcpyAsync(info, d_info.p, 8, cudaMemcpyDeviceToHost, c->stream));
+    HRN_CUDA(c, cudaStreamSynchronize(c->stream));
+    if (info[0] & kLineDispRow) return no("a node's displacement equations are not numbered in a row");
+    if (info[0] & kLineStressRow) return no("a node's stress equations are not numbered in a row");
+    if (info[0] & kLineStressOut) return no("a stress unknown lies outside the PML");
+    if (info[0] & kLineStressFixed) return no("the stresses of a PML node are constrained");
+    const int npn = total[0], nup = total[1], nun = total[1] + total[2], most = info[1];
     if (int64_t(3) * nun + int64_t(6) * npn != c->neq) return no("an equation belongs to no node or to several");
     if (most > kLineNb) return no("more than 32 elements share a node");
     if (nun == 0) return no("no displacement is free");
-    c->line_nun = nun;
     c->line_npn = npn;
-    std::vector<int32_t> &row = c->line_row;
-    row.assign(size_t(c->neq), 0);
-    for (int u = 0; u < nun; ++u)
-        for (int d = 0; d < 3; ++d) row[size_t(un_eq[u]) + d] = d * nun + u;
-    for (int p = 0; p < npn; ++p)
-        for (int d = 0; d < 6; ++d) row[size_t(pn_eq[p]) + d] = 3 * nun + d * npn + p;
-    std::vector<int32_t> ridx(std::max<size_t>(size_t(most) * nun, 1), -1);
-    for (int u = 0; u < nun; ++u)
-        for (int k = rptr[un_id[u]]; k < rptr[un_id[u] + 1]; ++k) {
-            const int e = rlist[k] / 27, q = rlist[k] % 27;
-            ridx[size_t(k - rptr[un_id[u]]) * nun + u] = 3 * c->nel_rd_e * q + e;
-        }
-    for (auto &p : rpt) p.y = unidx[p.x];
-    std::vector<int32_t> runode(rpt.size(), -1);   // by point, then element
-    for (int e = 0; e < c->nel_rd_e; ++e)
-        for (int q = 0; q < 27; ++q) runode[size_t(q) * c->nel_rd_e + e] = rpt[size_t(e) * 27 + q].y;
-    std::vector<int32_t> zidx(pidx);   // records of Z: PML nodes whose displacements are free
-    for (int j = 0; j < nj; ++j)
-        if (ubase[j] < 0) zidx[j] = -1;
-    DevBuf d_pn, d_pe, d_un, d_ue, d_zi, d_pi, d_fj, bad;
-    auto put = [&](DevBuf &b, const void *src, size_t bytes) -> int {
-        HRN_CUDA(c, b.alloc(std::max<size_t>(bytes, 16)));
-        if (bytes) HRN_CUDA(c, cudaMemcpyAsync(b.p, src, bytes, cudaMemcpyHostToDevice, c->stream));
-        return 0;
-    };
-    if (int rc = put(c->d_line_pnode, pnode.data(), pnode.size() * 8)) return rc;
-    if (int rc = put(c->d_line_unode, unode.data(), unode.size() * 16)) return rc;
-    if (int rc = put(c->d_line_ridx, ridx.data(), ridx.size() * 4)) return rc;
-    if (int rc = put(c->d_line_rpt, rpt.data(), rpt.size() * 8)) return rc;
-    if (int rc = put(c->d_line_runode, runode.data(), runode.size() * 4)) return rc;
-    if (int rc = put(c->d_line_row, row.data(), row.size() * 4)) return rc;
-    if (int rc = put(d_pn, pn_id.data(), pn_id.size() * 4)) return rc;
-    if (int rc = put(d_pe, pn_eq.data(), pn_eq.size() * 4)) return rc;
-    if (int rc = put(d_un, un_id.data(), un_id.size() * 4)) return rc;
-    if (int rc = put(d_ue, un_eq.data(), un_eq.size() * 4)) return rc;
-    if (int rc = put(d_zi, zidx.data(), zidx.size() * 4)) return rc;
-    if (int rc = put(d_pi, pidx.data(), pidx.size() * 4)) return rc;
+    c->line_nup = nup;
+    c->line_nun = nun;
+    auto room = [&](DevBuf &b, size_t bytes) { return b.alloc(std::max<size_t>(bytes, 16)); };
+    HRN_CUDA(c, room(c->d_line_pnode, size_t(npn) * 8));
+    HRN_CUDA(c, room(c->d_line_unode, size_t(nun) * 16));
+    HRN_CUDA(c, room(c->d_line_row, size_t(c->neq) * 4));
+    HRN_CUDA(c, room(d_pn, size_t(npn) * 4));
+    HRN_CUDA(c, room(d_pe, size_t(npn) * 4));
+    HRN_CUDA(c, room(d_un, size_t(nun) * 4));
+    HRN_CUDA(c, room(d_ue, size_t(nun) * 4));
+    HRN_CUDA(c, room(d_zi, size_t(nj) * 4));
+    HRN_CUDA(c, room(d_pi, size_t(nj) * 4));
+    HRN_CUDA(c, room(d_ui, size_t(nj) * 4));
+    k_line_lists<<<(nj + 255) / 256, 256, 0, c->stream>>>(
+        nj, npn, nup, nun, c->d_id.as<int32_t>(), flag, d_nrd.as<int32_t>(), c->d_line_pnode.as<int2>(), c->d_line_unode.as<int4>(),
+        d_pn.as<int32_t>(), d_pe.as<int32_t>(), d_un.as<int32_t>(), d_ue.as<int32_t>(), d_pi.as<int32_t>(), d_zi.as<int32_t>(),
+        d_ui.as<int32_t>(), c->d_line_row.as<int32_t>());
+    ++c->launches;
+    HRN_CUDA(c, room(c->d_line_ridx, size_t(most) * nun * 4));
+    HRN_CUDA(c, cudaMemsetAsync(c->d_line_ridx.p, 0xff, c->d_line_ridx.bytes, c->stream));   // -1: no entry
+    k_line_ridx<<<(nun + 255) / 256, 256, 0, c->stream>>>(nun, nrd, c->nel_pml_e, d_un.as<int32_t>(), c->d_nslot_ptr.as<int32_t>(),
+                                                          c->d_nslot.as<uint32_t>(), c->d_line_ridx.as<int32_t>());
+    ++c->launches;
+    HRN_CUDA(c, room(c->d_line_rpt, size_t(nrd) * 27 * 8));
+    HRN_CUDA(c, room(c->d_line_runode, size_t(nrd) * 27 * 4));
+    if (nrd > 0) {
+        k_line_points<<<unsigned((int64_t(nrd) * 27 + 255) / 256), 256, 0, c->stream>>>(
+            nrd, c->d_el_node.as<int32_t>() + size_t(c->nel_pml_e) * 27, d_ui.as<int32_t>(), c->d_line_rpt.as<int2>(), c->d_line_runode.as<int32_t>());
+        ++c->launches;
+    }
+    HRN_CUDA(c, cudaGetLastError());
     HRN_CUDA(c, bad.alloc(8));
     HRN_CUDA(c, cudaMemsetAsync(bad.p, 0, 8, c->stream));
     double j0 = 1.0;   // an inverse length of the PML's elements
@@ -351,11 +403,11 @@ static int line_tables(hrn_ctx *c)
     ++c->launches;
     HRN_CUDA(c, cudaGetLastError());
     const double *rg = c->d_el_geom.as<double>() + size_t(c->nel_pml_e) * 270;
-    int flag = 0;
-    HRN_CUDA(c, cudaMemcpyAsync(&flag, bad.p, 4, cudaMemcpyDeviceToHost, c->stream));
+    int unfit = 0;
+    HRN_CUDA(c, cudaMemcpyAsync(&unfit, bad.p, 4, cudaMemcpyDeviceToHost, c->stream));
     HRN_CUDA(c, cudaStreamSynchronize(c->stream));
-    if (flag == 1) return no("more than 32 nodes lie on the grid lines through one");
-    if (flag) return no("the PML's weights across a grid line vary along it (its elements are not aligned with the axes)");
+    if (unfit == 1) return no("more than 32 nodes lie on the grid lines through one");
+    if (unfit) return no("the PML's weights across a grid line vary along it (its elements are not aligned with the axes)");
     const int box = c->rd_box ? 1 : 0;
     const int64_t ng = int64_t(c->nel_rd_e) * (box ? 4 : 270);
     HRN_CUDA(c, c->d_line_rgeo.alloc(std::max<size_t>(size_t(ng), 1) * 8));
@@ -406,24 +458,26 @@ int line_ready(hrn_ctx *c, int *ok)
     if (c->line_epoch != c->epoch) {
         // sources, receivers or history rows on stress equations (none in an ordinary
         // set-up), and the state rows of the history and the receivers
-        const int first_stress = 3 * c->line_nun;
-        auto stress = [&](const std::vector<int32_t> &eqs) {
-            for (int32_t e : eqs)
-                if (c->line_row[e] >= first_stress) return 1;
-            return 0;
-        };
-        c->line_stress_src = stress(c->h_src_eq) | stress(c->h_eqdis);
-        c->line_stress_hist = stress(c->h_store_eq);
-        auto rows = [&](int n, const DevBuf &eq, DevBuf &out) -> int {
-            HRN_CUDA(c, out.alloc(std::max<size_t>(size_t(n) * 4, 16)));
+        DevBuf flags;   // sources and receivers, history
+        HRN_CUDA(c, flags.alloc(8));
+        HRN_CUDA(c, cudaMemsetAsync(flags.p, 0, 8, c->stream));
+        auto rows = [&](int n, const DevBuf &eq, DevBuf *out, int which) -> int {
+            if (out) HRN_CUDA(c, out->alloc(std::max<size_t>(size_t(n) * 4, 16)));
             if (n == 0) return 0;
-            k_line_rows<<<(n + 255) / 256, 256, 0, c->stream>>>(n, c->d_line_row.as<int32_t>(), eq.as<int32_t>(), out.as<int32_t>());
+            k_line_rows<<<(n + 255) / 256, 256, 0, c->stream>>>(n, 3 * c->line_nun, c->d_line_row.as<int32_t>(), eq.as<int32_t>(),
+                                                                out ? out->as<int32_t>() : nullptr, flags.as<int>() + which);
             ++c->launches;
             HRN_CUDA(c, cudaGetLastError());
             return 0;
         };
-        if (int rc = rows(c->nstore, c->d_store_eq, c->d_line_store_row)) return rc;
-        if (int rc = rows(c->nrec3, c->d_eqdis, c->d_line_rec_row)) return rc;
+        if (int rc = rows(c->nslot_f, c->d_fslot_eq, nullptr, 0)) return rc;
+        if (int rc = rows(c->nrec3, c->d_eqdis, &c->d_line_rec_row, 0)) return rc;
+        if (int rc = rows(c->nstore, c->d_store_eq, &c->d_line_store_row, 1)) return rc;
+        int h[2];
+        HRN_CUDA(c, cudaMemcpyAsync(h, flags.p, 8, cudaMemcpyDeviceToHost, c->stream));
+        HRN_CUDA(c, cudaStreamSynchronize(c->stream));
+        c->line_stress_src = h[0];
+        c->line_stress_hist = h[1];
         c->line_epoch = c->epoch;
     }
     *ok = 1;
