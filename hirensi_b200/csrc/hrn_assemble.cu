@@ -51,7 +51,7 @@ struct AsmArgs {
     const int32_t *elems;      // element ids of this colour
     int nel;
     const int32_t *inod, *id;
-    const double *xyz, *geom, *lam, *mu, *rho, *pml;
+    const double *geom, *lam, *mu, *rho;
     const double *pmlf;         // [nj][12] stretching factors of every node (k_asm_pml), kPastTop in [0] past the top
     const double *pmla;         // [nj] the factor a
     // values mode
@@ -584,15 +584,13 @@ int assemble_device(hrn_ctx *c, bool discover_pattern)
     AsmArgs A{};
     A.inod = c->d_inod.as<int32_t>();
     A.id = c->d_id.as<int32_t>();
-    A.xyz = c->d_xyz.as<double>();
     A.geom = c->d_asm_geom.as<double>();
     A.lam = c->d_lam.as<double>();
     A.mu = c->d_mu.as<double>();
     A.rho = c->d_rho.as<double>();
-    A.pml = c->d_pml.as<double>();
     if (!c->have_asm_pml) {
         HRN_CUDA(c, c->d_asm_pmlf.alloc(size_t(c->nj) * 13 * 8));
-        k_asm_pml<<<(c->nj + 255) / 256, 256, 0, c->stream>>>(c->nj, A.xyz, A.pml, c->d_asm_pmlf.as<double>(),
+        k_asm_pml<<<(c->nj + 255) / 256, 256, 0, c->stream>>>(c->nj, c->d_xyz.as<double>(), c->d_pml.as<double>(), c->d_asm_pmlf.as<double>(),
                                                               c->d_asm_pmlf.as<double>() + size_t(c->nj) * 12); ++c->launches;
         HRN_CUDA(c, cudaGetLastError());
         c->have_asm_pml = true;

@@ -346,6 +346,7 @@ int elem_stage(hrn_ctx *c, const void *stage_args, int stage, int adj, int acc, 
 bool elem_variant_valid(const hrn_ctx *c, int variant);
 // line-operator stage: 96, 97, 98 = up to 1, 2, 4 shots per thread (the most that divides
 // the shot count; 4 in FP32 only), so each serves any shot count
+constexpr int kLineCoef = 15;   // coefficient planes of a node
 inline bool is_line_variant(int v) { return v >= 96 && v <= 98; }
 bool line_reg_elements(const hrn_ctx *c);
 int line_ready(hrn_ctx *c, int *ok);

@@ -15,7 +15,6 @@ namespace hrn {
 
 constexpr int kLineNb = 32;        // most nodes that share a grid line through one node (13 on structured meshes)
 constexpr int kLineBuildThreads = 32;
-constexpr int kLineCoefPlanes = 15;
 // Entries below this share of their node's largest one are rounding residue of opposite
 // contributions (the one-sided derivatives at a node between two equal elements).
 constexpr double kLineDrop = 16 * 2.2204460492503131e-16;
@@ -387,7 +386,7 @@ static int line_tables(hrn_ctx *c)
     if (int rc = build_entries<T, 0>(c, npn, d_pn, d_zi, d_fj, &c->line_wd, c->d_line_didx, c->d_line_dcf, bad)) return rc;
     if (int rc = build_entries<T, 1>(c, c->line_nup, d_un, d_pi, d_fj, &c->line_wt, c->d_line_tidx, c->d_line_tcf, bad)) return rc;
     auto coef = [&](int n, int disp, const DevBuf &ids, const DevBuf &eqs, DevBuf &out) -> int {
-        HRN_CUDA(c, out.alloc(size_t(std::max(n, 1)) * kLineCoefPlanes * sizeof(T)));
+        HRN_CUDA(c, out.alloc(size_t(std::max(n, 1)) * kLineCoef * sizeof(T)));
         if (n == 0) return 0;
         k_line_coef<T><<<(n + 127) / 128, 128, 0, c->stream>>>(
             n, disp, ids.as<int32_t>(), eqs.as<int32_t>(), c->d_nslot_ptr.as<int32_t>(), c->d_nslot.as<uint32_t>(), c->nel_pml_e,

@@ -73,7 +73,7 @@ namespace hrn {
 //   9-11   -M^-1 EN (or EM) b, c, d
 //   12, 13 -M^-1 F j0 of the normal and the shear rows
 //   14     1 if a factor of G is not 0
-constexpr int kLineCoef = 15, kCoefDiag = 9, kCoefY = 12, kCoefYShear = 13, kCoefG = 14;
+constexpr int kCoefDiag = 9, kCoefY = 12, kCoefYShear = 13, kCoefG = 14;
 
 template <typename T>
 struct LineArgs {
