@@ -722,6 +722,8 @@ int hrn_set_receivers(hrn_ctx *c, int32_t nrec3, const int32_t *eqdis, const int
     if (!c) return HRN_EARG;
     ++c->epoch;
     if (nrec3 < 0 || (nrec3 > 0 && (!eqdis || !eqdis_map))) return set_error(c, HRN_EARG, "bad receiver arguments");
+    // a checkpointed forward keeps the traces of its own receivers only
+    if (c->ckpt > 0 && (nrec3 != c->nrec3 || !std::equal(c->h_eqdis.begin(), c->h_eqdis.end(), eqdis))) c->have_forward = false;
     c->nrec3 = nrec3;
     c->h_eqdis.assign(eqdis, eqdis + nrec3);
     c->h_eqdis_map.assign(eqdis_map, eqdis_map + nrec3);
@@ -872,6 +874,7 @@ static int upload_dis(hrn_ctx *c, const double *dis_meas, bool device_src = fals
     const size_t n = size_t(c->nshot) * c->nrec3 * (c->nstep + 1);
     if (!dis_meas) {
         if (n && !c->have_data) return set_error(c, HRN_ESTATE, "no measured data: pass dis_meas or call hrn_set_data");
+        if (n && c->d_dis.bytes != n * 8) return set_error(c, HRN_ESTATE, "the measured data are those of another number of receivers");
         return HRN_OK;
     }
     if (n == 0) return HRN_OK;

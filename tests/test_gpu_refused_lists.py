@@ -97,3 +97,41 @@ def test_refused_when_the_operator_comes(gpu_lib):
             x.set_variant(41, 41)
             x.forward()
         assert np.array_equal(s.history(0), r.history(0))
+
+
+def test_receivers_set_after_the_data_or_a_checkpointed_forward(gpu_lib):
+    """Data and traces are those of the receivers they came with: a longer list reads past neither."""
+    from hirensi_b200.capi import HrnError
+    from hirensi_b200.solver import Solver
+    p = tiny(nshot=1, nstep=20)
+    mesh = p["mesh"]
+    some, every = (p["eqdis"][:3], p["eqdis_map"][:3]), (p["eqdis"], p["eqdis_map"])
+    zero = np.zeros((1, len(p["eqdis"]), p["nstep"] + 1))
+    with Solver("fp64") as s:
+        s.set_mesh(mesh, RHO)
+        s.assemble(p["lam"], p["mu"])
+        s.set_history(mesh.store_eq)
+        s.set_shots(p["nstep"], p["dt"], p["src_eq"], p["src_b"], p["ftab"])
+        s.set_receivers(*some)
+        s.set_data(zero[:, :3])
+        s.set_variant(41, 41)
+        s.forward()
+        few = s.traces()
+        s.set_receivers(*every)             # the whole history: traces of any receivers
+        assert np.array_equal(s.traces()[:, :3], few)
+        for call in (lambda: s.misfit(None), lambda: s.adjoint_gradient(None)):
+            with pytest.raises(HrnError):
+                call()
+        assert s.misfit(zero) > 0.0
+        s.set_checkpointing(5)
+        s.forward()
+        s.set_receivers(*every)             # the same list changes nothing
+        assert np.array_equal(s.traces()[:, :3], few)
+        s.set_receivers(*some)
+        with pytest.raises(HrnError):
+            s.traces()
+        s.forward()
+        s.set_receivers(*every)
+        for call in (s.traces, lambda: s.misfit(zero), lambda: s.adjoint_gradient(zero)):
+            with pytest.raises(HrnError):
+                call()
