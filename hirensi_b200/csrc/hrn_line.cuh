@@ -262,7 +262,7 @@ __device__ __forceinline__ void add_history(const LineArgs<T> &L, int eq, int s0
 }
 
 // Threads of a block: one per node and SV shots, or 27 per regular-domain element and SV
-// shots.  Blocks of four to seven warps: with 224 to 256 threads for every shot count fewer
+// shots.  Blocks of three to seven warps: with 224 to 256 threads for every shot count fewer
 // blocks share an SM and their phases run in step (270 against 250 us, 40 x 40 x 20, FP32).
 template <int S, int SV>
 constexpr int line_threads()

@@ -1059,7 +1059,10 @@ static int autotune_lanes(hrn_ctx *c, StageArgs<T> a, T *X, T *Y, const TileArgs
         // other variant from about 70 thousand equations up; only on the smallest meshes, where
         // its two launches count, are the row-parallel kernels ahead (6 against 10 us a stage at
         // 8 thousand equations), and which of them depends on the lanes.  The tables of the
-        // others need not be built.
+        // others need not be built.  The same holds where the regular-domain elements are not
+        // boxes: with all 27 variants timed on distorted ones (1, 3, 4 and 8 shots, both
+        // precisions) the line variants are the three fastest at 70 thousand to 1.27 million
+        // equations, and 160, 161 or 96 is the fastest at 8 thousand.
         if (c->have_pattern) {
             if (c->neq < 100000) cand = {40, 80, 160, 41, 81, 161};
             else cand = {41, 81};

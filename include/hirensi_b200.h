@@ -129,7 +129,9 @@ int hrn_set_shots(hrn_ctx *ctx, int32_t nshot, int32_t nstep, double dt,
                   int32_t nsrc, const int32_t *src_eq, const double *src_b, const double *ftab);
 
 /* Receivers: EqDis (equations) and EqDis_MAP_U_Store_Numbers_Global (0-based
- * positions in the history), S4/IO_Parallel_Inversion.F90:116-133. */
+ * positions in the history), S4/IO_Parallel_Inversion.F90:116-133.  Resident data of another
+ * number of receivers have to be set again, and a checkpointed forward, which keeps the traces
+ * of its own receivers only, has to be run again for another list. */
 int hrn_set_receivers(hrn_ctx *ctx, int32_t nrec3, const int32_t *eqdis, const int32_t *eqdis_map);
 
 /* Shots of uneven record length and receiver count advanced in one batch.  The
