@@ -13,12 +13,6 @@ def test_first_reduction_under_capture(gpu_lib):
     from hirensi_b200.solver import Solver
     rng = np.random.default_rng(1)
     h = rng.standard_normal(100000)
-    # freed device memory with other contents: what the workspace may be cut from
-    for _ in range(2):
-        junk = [torch.full((1 << 18,), 7.0, dtype=torch.float64, device="cuda") for _ in range(4)]
-        torch.cuda.synchronize()
-        del junk
-        torch.cuda.empty_cache()
     x = torch.from_numpy(h).cuda()
     st = torch.cuda.Stream()
     torch.cuda.synchronize()
@@ -26,6 +20,13 @@ def test_first_reduction_under_capture(gpu_lib):
     p = C.c_void_p(x.data_ptr())
     rt = C.CDLL("libcudart.so.12")   # torch's, already loaded
     handle, graph = C.c_void_p(st.cuda_stream), C.c_void_p()
+    # freed blocks of the workspace's size with other contents: what it may be cut from
+    blocks = [C.c_void_p() for _ in range(2048)]
+    for b in blocks:
+        assert rt.cudaMalloc(C.byref(b), C.c_size_t(297 * 8)) == 0 and rt.cudaMemset(b, 7, C.c_size_t(297 * 8)) == 0
+    torch.cuda.synchronize()
+    for b in blocks[::2]:
+        assert rt.cudaFree(b) == 0
     with Solver("fp64") as s:
         s.set_stream(st.cuda_stream)
         assert rt.cudaStreamBeginCapture(handle, 2) == 0   # relaxed: allocations are allowed
@@ -40,3 +41,5 @@ def test_first_reduction_under_capture(gpu_lib):
             assert gpu_lib.hrn_vec_dot(s.h, x.numel(), p, p, C.byref(out)) == 0
             ref = float(np.dot(h * scale, h * scale))
             assert abs(out.value - ref) <= 1e-13 * ref
+    for b in blocks[1::2]:
+        assert rt.cudaFree(b) == 0
